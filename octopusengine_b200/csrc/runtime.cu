@@ -850,7 +850,14 @@ void enqueue_effects(oct_scene* s, float dt, cudaStream_t st) {
 
 // One GPU_VBD::step (octopus/src/GPU/VBD/GPU_VBD.cu:38-61) of one scene with the reference's
 // launch structure: predictor, iterations x (one launch per colour [+ commit] + constraints
-// [+ Chebyshev]), velocity update.
+// [+ Chebyshev]), velocity update.  The fixation runs in the sub-step's first iteration only:
+// it puts the fixed nodes, which the predictor moved, on their target and clears their mask,
+// and from then on nothing in the sub-step moves them (sweeps, effects and the box skip masked
+// nodes, Chebyshev mixes equal values), so writing the same values again every iteration was
+// one launch in each for nothing: 81-node P1 frame of 20 iterations 339 -> 314 us, P1 of 98,304
+// elements 455 -> 424 us.  Multigrid's prolongation moves fixed mid nodes, so it keeps the launch;
+// so do batches, where it joins the groups' branches (without it 14.30 -> 14.46 ms per frame of
+// 16 mixed scenes).
 void vbd_substep(oct_scene* s, float dt) {
     Range range("vbd_substep");
     oct_ctx* c = s->ctx;
@@ -906,7 +913,7 @@ void vbd_substep(oct_scene* s, float dt) {
             c->launches++;
             if (!s->in_place) { launch_commit(s->d_scene, s->d_vwork + b, n, st); c->launches++; }
         }
-        if (s->n_fixed) { launch_constraints(s->d_scene, s->d_fwork, s->n_fwork, 0, st); c->launches++; }
+        if (s->n_fixed && (j == 0 || s->mg_sub)) { launch_constraints(s->d_scene, s->d_fwork, s->n_fwork, 0, st); c->launches++; }
         enqueue_effects(s, dt, st);
         if (s->box) { launch_constraints(s->d_scene, s->d_nwork, s->n_nwork, 1, st); c->launches++; }
         if (cheb) {
