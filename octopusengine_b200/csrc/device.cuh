@@ -61,6 +61,7 @@ struct SceneDev {
     const int* topo;    // n_elements * NE
     const float4* eq;   // n_elements * NQ * 3
     const int* vids;    // n_nodes, colour-sorted
+    const int4* slots;  // the same slots with their owners: node, first owner, owner count, 0
     const int* own_off; // n_nodes + 1, slot order
     const int* owners;  // packed (eid << 5) | r
     const int* fixed;   // n_fixed node ids
@@ -96,18 +97,18 @@ struct XWork {
 constexpr int kStatusTimeout = 1;      // a bounded wait gave up on this scene's work
 constexpr int kStatusNonFinite = 2;    // a node's position or velocity became NaN / Inf
 
-// One unit of colour work: `count` consecutive colour slots of one scene.  With a fixed
-// number of lanes per vertex an item fills one block (128 / lanes slots); in the packed
+// One unit of colour work: `count` consecutive colour slots of one scene.  With a number of
+// lanes per vertex an item fills one block (128 / lanes slots); in the packed
 // mapping an item fills one warp (one lane per (vertex, owner) pair, at most 32 pairs) and
 // pair_base is the owner-CSR offset of its first slot.
-struct VWork {
+struct alignas(16) VWork {
     int scene;
     int slot_begin;
     int count;
+    int lanes;        // lane-group items: lanes per vertex
     int pair_base;
     unsigned heads;   // packed items: bit p set when pair p starts a new vertex
     int n_pairs;      // packed items: number of (vertex, owner) pairs
-    int tpv;          // lane-group items: lanes per vertex of this item; 0 = the launch's
     int pad1;
 };
 

@@ -340,7 +340,7 @@ __device__ __forceinline__ void p2_jacobian(const float* ux, const float* uy, co
 template <int E, int MAT>
 __device__ __forceinline__ void element_terms(const float* ux, const float* uy, const float* uz, int r, float4 A, float4 B,
                                               float4 C, const float4* __restrict__ rec, bool affine,
-                                              const float* __restrict__ s_dN, bool mixed, float acc[9], float cmp[9],
+                                              const float* __restrict__ s_dN, bool mixed, float acc[9], float cmp[3],
                                               unsigned long long stream) {
     constexpr int NE = ElemT<E>::NE, NQ = ElemT<E>::NQ;
     float fs[3] = {0.f, 0.f, 0.f};   // CompensatePerElement: the element's force over its points
@@ -412,7 +412,7 @@ __device__ __forceinline__ void element_terms(const float* ux, const float* uy, 
 // Owner given as a packed (element, local node) id: topology and records from global memory.
 template <int E, int MAT>
 __device__ __forceinline__ void owner_terms(const SceneDev& S, int packed, const float* __restrict__ s_dN, bool mixed,
-                                            float acc[9], float cmp[9]) {
+                                            float acc[9], float cmp[3]) {
     constexpr int NE = ElemT<E>::NE;
     const int eid = packed >> kOwnerShift, r = packed & ((1 << kOwnerShift) - 1);
     const int* __restrict__ tp = S.topo + (size_t)eid * NE;
@@ -454,7 +454,7 @@ template <int NE> __device__ __forceinline__ int entry_rec(const float* en) {
 // Owner given as an entry (EntryLayout), staged in shared memory or held in registers.
 template <int E, int MAT>
 __device__ __forceinline__ void entry_terms(const SceneDev& S, const float* __restrict__ en, const float* __restrict__ s_dN,
-                                            bool mixed, float acc[9], float cmp[9]) {
+                                            bool mixed, float acc[9], float cmp[3]) {
     constexpr int NE = ElemT<E>::NE, NQ = ElemT<E>::NQ;
     const unsigned long long keep = policy_keep(), stream = policy_stream();
     if constexpr (NE == 4) {   // P1: own node first, the corner's record holds G_j of the other three
@@ -547,8 +547,7 @@ __device__ __forceinline__ V3 newton_step(const float acc[9], float4 uu, float4 
 }
 
 // ------------------------------------------------------------------------ colour kernels
-// Per-vertex epilogue. mode 0: VBD solve; mode 1: VBD residual (writes |r| reductions);
-// mode 2: explicit force (kernel_fem_eval_force, GPU_FEM_Explicit.cu:5-64).
+// Per-vertex epilogue. mode 0: VBD solve; mode 1: VBD residual (writes |r| reductions).
 __device__ __forceinline__ void vertex_epilogue(const SceneDev& S, int vid, const float acc[9], int mode, const StepParams& P,
                                                 double* red) {
     const float4 uu = S.u[vid], ul = S.u_last[vid], yy = S.y[vid];
@@ -556,7 +555,7 @@ __device__ __forceinline__ void vertex_epilogue(const SceneDev& S, int vid, cons
         const V3 d = newton_step(acc, uu, ul, yy, S.damping, P.inv_dt, S.precision);
         const float4 un = make_float4(uu.x + d.x, uu.y + d.y, uu.z + d.z, uu.w);
         if (P.in_place) S.u[vid] = un; else S.u_new[vid] = un;
-    } else if (mode == 1) {
+    } else {
         // kernel_vbd_compute_residual (GPU_VBD_FEM.cu:482-546)
         const float kd = S.damping * P.inv_dt, mh2 = yy.w * P.inv_dt * P.inv_dt;
         const float dx = uu.x - ul.x, dy = uu.y - ul.y, dz = uu.z - ul.z;
@@ -571,16 +570,6 @@ __device__ __forceinline__ void vertex_epilogue(const SceneDev& S, int vid, cons
             unsigned long long* mx = reinterpret_cast<unsigned long long*>(red + 1);
             atomicMax(mx, (unsigned long long)__double_as_longlong(nr));
         }
-    } else {
-        // f = sum(-P g V) - k_d H v, written to u_new (the force buffer of the explicit solver)
-        const float4 vv = S.v[vid];
-        const float kd = S.damping;
-        float4 f;
-        f.x = acc[0] - kd * (acc[3] * vv.x + acc[4] * vv.y + acc[5] * vv.z);
-        f.y = acc[1] - kd * (acc[4] * vv.x + acc[6] * vv.y + acc[7] * vv.z);
-        f.z = acc[2] - kd * (acc[5] * vv.x + acc[7] * vv.y + acc[8] * vv.z);
-        f.w = 0.f;
-        S.u_new[vid] = f;
     }
 }
 
@@ -666,7 +655,7 @@ __global__ void __launch_bounds__(kBlock, MinBlocks<E>::value) k_vertex_packed(c
         bool active = false;
         if (lane < wk.n_pairs) {
             vid = entry_node(en, entry_r<NE>(en));
-            active = mode == 2 || S.mask[vid] != 0;
+            active = S.mask[vid] != 0;
         }
         float acc[9], cmp[9];
 #pragma unroll
@@ -707,7 +696,7 @@ __global__ void __launch_bounds__(kBlock, MinBlocks<E>::value) k_vertex_packed(c
 template <int E> constexpr int packed_smem_bytes() { return (kBlock / 32) * 2 * 32 * EntryLayout<ElemT<E>::NE>::kWords * 4; }
 
 // ------------------------------------------------------------------------ colour kernel
-// mode 0: VBD solve; mode 1: VBD residual (r into u_new, |r| reductions); mode 2: explicit force.
+// mode 0: VBD solve; mode 1: VBD residual (r into u_new, |r| reductions).
 // Resident blocks per SM the lane-group kernel is compiled for: P2 and Q1 are held to 128
 // registers (4 blocks, 16 warps per SM; ptxas spills a few bytes), P1 to 80.
 #ifndef OCTB_P2_MIN_BLOCKS
@@ -723,72 +712,87 @@ template <int E> struct LaneMinBlocks {
     static constexpr int value = E == 3 ? OCTB_P1_MIN_BLOCKS : (E == 6 ? OCTB_Q1_MIN_BLOCKS : (E == 7 ? OCTB_P2_MIN_BLOCKS : 1));
 };
 
+// A colour launch of one scene is a chain of dependent loads more than it is work: work item,
+// scene pointers, vertex slot, owner entry, node displacements, then the solve's own state.  All
+// of it up to the first owner entry is data that no kernel of a step writes, so it is loaded
+// before pdl_wait(), under the previous colour's tail; after the wait only the gathers, the
+// arithmetic and the store are left.  The slot (node, first owner, owner count) is one 16-byte
+// load, and the state the solve needs is prefetched into L1 while the owners are evaluated.
 template <int E, int MAT>
 __global__ void __launch_bounds__(kBlock, LaneMinBlocks<E>::value) k_vertex(const SceneDev* __restrict__ scenes, const VWork* __restrict__ work,
-                                                   int n_work, int tpv, int mode, StepParams P, double* red) {
+                                                   int n_work, int mode, StepParams P, double* red) {
     constexpr int NE = ElemT<E>::NE, NQ = ElemT<E>::NQ;
+    constexpr int EW = EntryLayout<NE>::kWords;
     __shared__ __align__(128) float s_dN[((NQ * NE * 3 + 3) / 4) * 4];
     __shared__ __align__(8) unsigned long long s_mbar;
+    const int lane = threadIdx.x & 31;
+    const unsigned long long stream = policy_stream();
+    int scene, t, glane, o, oe, vid;
+    bool valid;
+    float4 nxt[EW / 4];
+    auto fetch = [&](int w) {   // this lane's part of item w, up to its first owner entry
+        const int4 wk = __ldg(reinterpret_cast<const int4*>(work + w));   // scene, slot_begin, count, lanes
+        scene = wk.x;
+        t = wk.w;                            // lanes per vertex of this item (block-uniform)
+        glane = lane & (t - 1);              // lane within the vertex group
+        const int group = threadIdx.x >> (__ffs(t) - 1);   // vertex index within the block
+        const SceneDev& S = scenes[scene];
+        valid = group < wk.z;
+        const int4 sl = valid ? __ldg(S.slots + wk.y + group) : make_int4(0, 0, 0, 0);
+        vid = sl.x;
+        o = sl.y + glane;
+        oe = sl.y + sl.z;
+        if (S.ent && o < oe) {
+#pragma unroll
+            for (int j = 0; j < EW / 4; ++j) nxt[j] = ld_hint(S.ent + (size_t)o * (EW / 4) + j, stream);
+        }
+    };
+    int w = blockIdx.x;
+    fetch(w);
     stage_table(s_dN, gdN<E>(), NQ * NE * 3, &s_mbar, P.error);
     pdl_wait();
-
-    const int lane = threadIdx.x & 31;
-    for (int w = blockIdx.x; w < n_work; w += gridDim.x) {
-        const VWork wk = work[w];
-        const int t = wk.tpv ? wk.tpv : tpv;    // lanes per vertex of this item (block-uniform)
-        const int glane = lane & (t - 1);        // lane within the vertex group
-        const int group = threadIdx.x / t;       // vertex index within the block
-        const SceneDev& S = scenes[wk.scene];
-        const bool valid = group < wk.count;
-        const int slot = wk.slot_begin + group;
-        int vid = 0;
-        bool active = false;
-        if (valid) {
-            vid = __ldg(S.vids + slot);
-            active = mode == 2 || S.mask[vid] != 0;
+    while (true) {
+        const SceneDev& S = scenes[scene];
+        const bool active = valid && S.mask[vid] != 0;
+        if (active && glane == 0) {
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(S.u_last + vid));
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(S.y + vid));
         }
-        float acc[9], cmp[9];
+        float acc[9], cmp[3];
 #pragma unroll
-        for (int k = 0; k < 9; ++k) { acc[k] = 0.f; cmp[k] = 0.f; }
+        for (int k = 0; k < 9; ++k) acc[k] = 0.f;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) cmp[k] = 0.f;
         const bool mixed = S.precision != 0;
-        if (active) {
-            const int ob = __ldg(S.own_off + slot), oe = __ldg(S.own_off + slot + 1);
-            if (S.ent) {
-                // owner entries (contiguous per vertex): load the next one while this one computes
-                constexpr int EW = EntryLayout<NE>::kWords;
-                const float4* base = S.ent;
-                const unsigned long long stream = policy_stream();
-                int o = ob + glane;
-                float4 nxt[EW / 4];
+        if (S.ent) {
+            // owner entries (contiguous per vertex): load the next one while this one computes
+            const float4* base = S.ent;
+            while (o < oe) {
+                float4 cur[EW / 4];
+#pragma unroll
+                for (int j = 0; j < EW / 4; ++j) cur[j] = nxt[j];
+                o += t;
                 if (o < oe) {
 #pragma unroll
                     for (int j = 0; j < EW / 4; ++j) nxt[j] = ld_hint(base + (size_t)o * (EW / 4) + j, stream);
                 }
-                while (o < oe) {
-                    float4 cur[EW / 4];
-#pragma unroll
-                    for (int j = 0; j < EW / 4; ++j) cur[j] = nxt[j];
-                    const int on = o + t;
-                    if (on < oe) {
-#pragma unroll
-                        for (int j = 0; j < EW / 4; ++j) nxt[j] = ld_hint(base + (size_t)on * (EW / 4) + j, stream);
-                    }
-                    entry_terms<E, MAT>(S, reinterpret_cast<const float*>(cur), s_dN, mixed, acc, cmp);
-                    o = on;
-                }
-            } else {
-                for (int o = ob + glane; o < oe; o += t) owner_terms<E, MAT>(S, __ldg(S.owners + o), s_dN, mixed, acc, cmp);
+                entry_terms<E, MAT>(S, reinterpret_cast<const float*>(cur), s_dN, mixed, acc, cmp);
             }
-            if (mixed) {
+        } else {
+            for (; o < oe; o += t) owner_terms<E, MAT>(S, __ldg(S.owners + o), s_dN, mixed, acc, cmp);
+        }
+        if (mixed) {
 #pragma unroll
-                for (int k = 0; k < 3; ++k) acc[k] -= cmp[k];
-            }
+            for (int k = 0; k < 3; ++k) acc[k] -= cmp[k];
         }
         for (int off = t >> 1; off > 0; off >>= 1) {
 #pragma unroll
             for (int k = 0; k < 9; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], off);
         }
         if (active && glane == 0) vertex_epilogue(S, vid, acc, mode, P, red);
+        w += gridDim.x;
+        if (w >= n_work) break;
+        fetch(w);
     }
     pdl_trigger();   // after the sweep: the next launch overlaps this kernel's tail only
 }
@@ -1793,7 +1797,7 @@ void vertex_dispatch(const SceneDev* scenes, const VWork* work, int n_work, int 
     int cap = grid_cap<E, MAT, false>();
     if (cap <= 0) cap = 148 * 4;
     const int grid = n_work < cap ? n_work : cap;
-    launch_pdl(k_vertex<E, MAT>, grid, kBlock, 0, st, scenes, work, n_work, tpv, mode, P, red);
+    launch_pdl(k_vertex<E, MAT>, grid, kBlock, 0, st, scenes, work, n_work, mode, P, red);
 }
 
 template <int E>

@@ -11,7 +11,7 @@ cudaError_t upload_shape_tables_fp64(int element, const double* dN, int n, const
 // Caches the persistent grid size of the vertex kernel for (element, material); call
 // outside stream capture.
 void prepare_vertex(int element, int material);
-// mode 0: VBD solve, 1: VBD residual (red[0] += |r|, red[1] = max |r|), 2: explicit force
+// mode 0: VBD solve, 1: VBD residual (red[0] += |r|, red[1] = max |r|)
 void launch_vertex(int element, int material, const SceneDev* scenes, const VWork* work, int n_work, int tpv, int mode,
                    const StepParams& P, double* red, cudaStream_t st);
 void launch_commit(const SceneDev* scenes, const VWork* work, int n_work, cudaStream_t st);

@@ -259,18 +259,52 @@ oct_status ensure_tables(oct_ctx* c, int element) {
 // P1 (20-24 owners) with 8 lanes instead of 4, 0.221 -> 0.298 ms.
 constexpr int kOwnersPerLane = 8;
 
+// measured_tpv, used when the description leaves the lanes at 0
+int measured_tpv(int element);
+
+// Lanes of one scene's colour.  least: as above.  width: with the default mapping, the power of
+// two nearest the colour's owners per vertex (about one owner per lane); else least.
+struct ColourLanes {
+    int least = 1, width = 1;
+    int at(int div) const { return std::max(least, width / div); }
+};
+ColourLanes colour_lanes(int element, int tpv, int begin, int end, const std::vector<int32_t>& own_off) {
+    ColourLanes l;
+    l.least = l.width = tpv;
+    if (tpv <= 0 || end <= begin) return l;
+    const int64_t n = end - begin, pairs = (int64_t)own_off[end] - own_off[begin];
+    while (l.least < 32 && pairs > (int64_t)kOwnersPerLane * l.least * n) l.least <<= 1;
+    l.width = l.least;
+    if (tpv != measured_tpv(element)) return l;
+    while (l.width < 32 && 2 * pairs >= 3 * (int64_t)l.width * n) l.width <<= 1;
+    return l;
+}
+
+// What a launch whose vertices take `full` lanes at full width divides the widths by: the
+// smallest power of two that leaves at most kLaunchLanes lanes.  A launch with few vertices
+// waits for the chain of owners of its longest lane, so it gets about one owner per lane; one
+// that fills the GPU (75,000 lanes of the P2 and Q1 kernels are resident, 113,000 of P1) only
+// pays for idle lanes and reductions.  Frame of one scene with least lanes / 30,000 / 50,000 /
+// 80,000: P2 98,304 elements 5.64 / 5.18 / 4.31 / 4.74 ms, P1 98,304 elements 0.405 / 0.409 /
+// 0.360 / 0.377 ms, Q1 2,233 elements 0.90 / 0.75 / 0.75 / 0.75 ms; 16 mixed scenes 13.9 / 11.8 /
+// 10.5 / 11.1 ms; one iteration of 200 mixed scenes of 430 nodes 132 / 97 / 80 / 80 us, of 64
+// scenes of 30,000 nodes 624 / 618 / 615 / 616 us.
+int lane_div(int64_t full) {
+    constexpr int64_t kLaunchLanes = 50000;
+    int div = 1;
+    while (div < 32 && full > kLaunchLanes * div) div <<= 1;
+    return div;
+}
+
 // Split [begin, end) slots into work items for one scene: block-sized items of 128 / t slots
-// (t lanes per vertex, the colour's count from tpv and kOwnersPerLane), or (tpv == 0) warp
-// items packing whole vertices up to 32 (vertex, owner) pairs and at most 31 slots.
-void append_vwork(std::vector<VWork>& out, int scene, int begin, int end, int tpv, const std::vector<int32_t>& own_off) {
+// (l, div as above), or (tpv == 0) warp items packing whole vertices up to 32 (vertex, owner)
+// pairs and at most 31 slots.
+void append_vwork(std::vector<VWork>& out, int scene, int begin, int end, int tpv, ColourLanes l, int div,
+                  const std::vector<int32_t>& own_off) {
     if (tpv > 0) {
-        int t = tpv;
-        if (end > begin) {
-            const int64_t pairs = (int64_t)own_off[end] - own_off[begin];
-            while (t < 32 && pairs > (int64_t)kOwnersPerLane * t * (end - begin)) t <<= 1;
-        }
-        const int vpb = kBlockThreads / t;
-        for (int s = begin; s < end; s += vpb) out.push_back({scene, s, std::min(vpb, end - s), 0, 0u, 0, t, 0});
+        const int t = l.at(div), vpb = kBlockThreads / t;
+        for (int s = begin; s < end; s += vpb)
+            out.push_back({scene, s, std::min(vpb, end - s), t, 0, 0u, 0, 0});
         return;
     }
     int s = begin;
@@ -282,7 +316,7 @@ void append_vwork(std::vector<VWork>& out, int scene, int begin, int end, int tp
             pairs += own_off[s + n + 1] - own_off[s + n];
             ++n;
         }
-        out.push_back({scene, s, n, own_off[s], heads, pairs, 0, 0});
+        out.push_back({scene, s, n, 0, own_off[s], heads, pairs, 0});
         s += n;
     }
 }
@@ -335,7 +369,9 @@ oct_status build_vertex_work(oct_scene* s) {
     std::vector<VWork> vw;
     s->vwork_off.assign(1, 0);
     for (int k = 0; k + 1 < (int)s->color_off.size(); ++k) {
-        append_vwork(vw, 0, s->color_off[k], s->color_off[k + 1], s->tpv, s->own_off);
+        const int begin = s->color_off[k], end = s->color_off[k + 1];
+        const ColourLanes l = colour_lanes(s->element, s->tpv, begin, end, s->own_off);
+        append_vwork(vw, 0, begin, end, s->tpv, l, lane_div((int64_t)l.width * (end - begin)), s->own_off);
         s->vwork_off.push_back((int)vw.size());
     }
     return upload(s->ctx, s->mem, s->d_vwork, vw);
@@ -684,6 +720,11 @@ oct_status build_scene(oct_ctx* c, const oct_scene_desc* d, oct_scene* s) {
     if ((st = upload(c, s->mem, maskd, mask)) || (st = upload(c, s->mem, topod, topo)) || (st = upload(c, s->mem, eqd, eq)) ||
         (st = upload(c, s->mem, vidsd, slot_vids)) || (st = upload(c, s->mem, offd, own_off)) || (st = upload(c, s->mem, ownd, owners)))
         return st;
+    std::vector<int4> slots(N);
+    for (int sl = 0; sl < N; ++sl) slots[sl] = make_int4(slot_vids[sl], own_off[sl], own_off[sl + 1] - own_off[sl], 0);
+    int4* slotd;
+    if ((st = upload(c, s->mem, slotd, slots))) return st;
+    h.slots = slotd;
     int* fgd = nullptr;
     if (s->n_fixed && ((st = upload(c, s->mem, fixd, s->fixed)) || (st = upload(c, s->mem, fgd, s->fixed_group)))) return st;
     if ((st = upload(c, s->mem, s->d_fix, std::vector<float>(s->fix_host, s->fix_host + kFixGroups * 16)))) return st;
@@ -1076,7 +1117,7 @@ oct_status oct_scene_footprint(const oct_scene_desc* d, size_t* bytes) {
     const int ne = element_nodes(d->element), nq = element_quadrature(d->element);
     if (ne < 0 || d->n_nodes <= 0 || d->n_elements <= 0) return OCT_EINVAL;
     const size_t N = d->n_nodes, E = d->n_elements;
-    size_t b = N * (6 * sizeof(float4) + 3 * sizeof(int)) + (d->rho > 0.f ? 2 * N * sizeof(float4) : 0);
+    size_t b = N * (7 * sizeof(float4) + 3 * sizeof(int)) + (d->rho > 0.f ? 2 * N * sizeof(float4) : 0);
     b += E * ne * sizeof(int) * 2 + E * nq * 3 * sizeof(float4);   // topology, owners, quadrature records
     b += E * ne * (size_t)entry_words(ne) * sizeof(float);                  // owner entries
     b += (ne == 4 ? 4 : 1) * E * 3 * sizeof(float4);                        // distinct records, at most
@@ -1587,6 +1628,7 @@ oct_status oct_batch_create(oct_ctx* c, oct_scene* const* scenes, int n, oct_bat
     std::map<std::pair<std::pair<int, int>, std::pair<int, int>>, int> gid;
     std::vector<std::vector<std::vector<VWork>>> gwork;   // group -> colour -> items
     std::vector<std::vector<std::vector<XWork>>> gxwork;  // XPBD: group -> colour -> items
+    std::vector<std::vector<int>> members;                // VBD: group -> its scenes
     size_t off = 0;
     for (int i = 0; i < n; ++i) {
         oct_scene* s = scenes[i];
@@ -1632,10 +1674,28 @@ oct_status oct_batch_create(oct_ctx* c, oct_scene* const* scenes, int n, oct_bat
             g.element = s->element; g.material = s->material; g.tpv = s->tpv; g.in_place = s->in_place;
             b->groups.push_back(g);
             gwork.emplace_back();
+            members.emplace_back();
         }
-        auto& cw = gwork[it->second];
-        if ((int)cw.size() < s->n_colors) cw.resize(s->n_colors);
-        for (int k = 0; k < s->n_colors; ++k) append_vwork(cw[k], i, s->color_off[k], s->color_off[k + 1], s->tpv, s->own_off);
+        members[it->second].push_back(i);
+    }
+    for (size_t g = 0; g < members.size(); ++g) {   // VBD: the items of each group's colours, across its scenes
+        auto& cw = gwork[g];
+        for (int i : members[g]) cw.resize(std::max(cw.size(), (size_t)scenes[i]->n_colors));
+        for (int k = 0; k < (int)cw.size(); ++k) {
+            std::vector<ColourLanes> l;
+            int64_t full = 0;
+            for (int i : members[g]) {
+                const oct_scene* s = scenes[i];
+                const bool has = k < s->n_colors;
+                l.push_back(has ? colour_lanes(s->element, s->tpv, s->color_off[k], s->color_off[k + 1], s->own_off) : ColourLanes());
+                if (has) full += (int64_t)l.back().width * (s->color_off[k + 1] - s->color_off[k]);
+            }
+            for (size_t m = 0; m < members[g].size(); ++m) {
+                const oct_scene* s = scenes[members[g][m]];
+                if (k < s->n_colors)
+                    append_vwork(cw[k], members[g][m], s->color_off[k], s->color_off[k + 1], s->tpv, l[m], lane_div(full), s->own_off);
+            }
+        }
     }
     b->state_off.push_back(off);
     std::vector<VWork> all;
