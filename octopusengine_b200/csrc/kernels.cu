@@ -160,6 +160,15 @@ __device__ __forceinline__ float4 ld_hint(const float4* a, unsigned long long po
         : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(a), "l"(pol));
     return v;
 }
+// A node displacement.  COH: in a kernel whose own blocks write displacements between grid
+// barriers (k_vbd_substep) the load must not use the read-only path.
+template <bool COH> __device__ __forceinline__ float4 ld_node(const float4* a, unsigned long long pol) {
+    if constexpr (!COH) return ld_hint(a, pol);
+    float4 v;
+    asm volatile("ld.global.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(a), "l"(pol) : "memory");
+    return v;
+}
 __device__ __forceinline__ int ld_hint(const int* a, unsigned long long pol) {
     int v;
     asm("ld.global.nc.L2::cache_hint.s32 %0, [%1], %2;" : "=r"(v) : "l"(a), "l"(pol));
@@ -452,16 +461,16 @@ template <int NE> __device__ __forceinline__ int entry_rec(const float* en) {
 }
 
 // Owner given as an entry (EntryLayout), staged in shared memory or held in registers.
-template <int E, int MAT>
+template <int E, int MAT, bool COH = false>
 __device__ __forceinline__ void entry_terms(const SceneDev& S, const float* __restrict__ en, const float* __restrict__ s_dN,
                                             bool mixed, float acc[9], float cmp[3]) {
     constexpr int NE = ElemT<E>::NE, NQ = ElemT<E>::NQ;
     const unsigned long long keep = policy_keep(), stream = policy_stream();
     if constexpr (NE == 4) {   // P1: own node first, the corner's record holds G_j of the other three
-        const float4 u0 = ld_hint(&S.u[entry_node(en, 0)], keep);
-        const float4 u1 = ld_hint(&S.u[entry_node(en, 1)], keep);
-        const float4 u2 = ld_hint(&S.u[entry_node(en, 2)], keep);
-        const float4 u3 = ld_hint(&S.u[entry_node(en, 3)], keep);
+        const float4 u0 = ld_node<COH>(&S.u[entry_node(en, 0)], keep);
+        const float4 u1 = ld_node<COH>(&S.u[entry_node(en, 1)], keep);
+        const float4 u2 = ld_node<COH>(&S.u[entry_node(en, 2)], keep);
+        const float4 u3 = ld_node<COH>(&S.u[entry_node(en, 3)], keep);
         const float4* R = S.rtab + 3 * (size_t)entry_rec<NE>(en);
         const float4 R0 = ld_hint(R, keep), R1 = ld_hint(R + 1, keep), R2 = ld_hint(R + 2, keep);
         const V3 d1 = xyz(u1) - xyz(u0), d2 = xyz(u2) - xyz(u0), d3 = xyz(u3) - xyz(u0);
@@ -488,7 +497,7 @@ __device__ __forceinline__ void entry_terms(const SceneDev& S, const float* __re
     float ux[NE], uy[NE], uz[NE];
 #pragma unroll
     for (int i = 0; i < NE; ++i) {
-        const float4 t = ld_hint(&S.u[entry_node(en, i)], keep);
+        const float4 t = ld_node<COH>(&S.u[entry_node(en, i)], keep);
         ux[i] = t.x; uy[i] = t.y; uz[i] = t.z;
     }
     const int r = entry_r<NE>(en), rec = entry_rec<NE>(en);
@@ -591,7 +600,7 @@ __device__ __forceinline__ bool mbar_wait(unsigned mb, unsigned phase, long limi
 // the next item's entries arrive while the current item computes, leaving the node-
 // displacement gathers as the only dependent global loads.
 // Resident blocks per SM each element type is compiled for (register cap without spills).
-template <int E> struct MinBlocks { static constexpr int value = E == 3 ? 8 : (E == 7 ? 5 : (E == 6 ? 4 : (E == 8 ? 4 : 2))); };
+template <int E> struct MinBlocks { static constexpr int value = E == 3 ? 8 : (E == 7 ? 5 : 4); };
 
 template <int E, int MAT>
 __global__ void __launch_bounds__(kBlock, MinBlocks<E>::value) k_vertex_packed(const SceneDev* __restrict__ scenes,
@@ -694,6 +703,252 @@ __global__ void __launch_bounds__(kBlock, MinBlocks<E>::value) k_vertex_packed(c
 }
 
 template <int E> constexpr int packed_smem_bytes() { return (kBlock / 32) * 2 * 32 * EntryLayout<ElemT<E>::NE>::kWords * 4; }
+
+// ------------------------------------------------------------------------ point lanes
+// The packed mapping of the many-point elements (P3 11 points x 20 nodes, Q2 27 x 27).  One lane
+// per (vertex, owner) pair ran all points in series: a Q2 colour of a 2,048-element beam holds
+// about 2,000 pairs, 64 warps on 148 SMs, each 10,000 instructions deep.  Here LP lanes share a
+// pair, three points each (P3 4 lanes, Q2 9), so a launch has LP times the lanes and a chain a
+// quarter to a ninth as long, for the same work per pair or less:
+//   Q2: the lane's three points share (y, z), and the basis is a tensor product, so the node
+//       displacements are contracted along z, then y (18 + 9 values per column of nodes), then
+//       along x at the three points: 324 FMAs where three dense contractions took 729;
+//   P3: the dense contraction per point, its dN row read from shared memory.
+// A pair's nodes are gathered once by its lanes into shared memory.  A block takes whole vertices
+// up to its number of pair slots; a pair's lanes are summed first, then each vertex's pairs in
+// owner order (compensated in mixed precision), so the result does not depend on the packing.  A
+// vertex with more owners than slots takes an item of its own in several rounds.
+template <int E> struct PointLanes;
+template <> struct PointLanes<8> { static constexpr int LP = 4, PP = 3, kThreads = 192, kRow = 21, kMinBlocks = 2; };
+template <> struct PointLanes<9> { static constexpr int LP = 9, PP = 3, kThreads = 256, kRow = 27, kMinBlocks = 2; };
+template <int E> constexpr int point_slots() { return PointLanes<E>::kThreads / 32 * (32 / PointLanes<E>::LP); }
+
+// 1-D quadratic basis on {-1, 0, 1} at the Gauss points -sqrt(3/5), 0, sqrt(3/5) (index 0 1 2).
+constexpr double kSqrt35 = 0.77459666924148337704;
+__host__ __device__ constexpr float q2_n(int point, int node) {
+    const double s = (point - 1) * kSqrt35;
+    return (float)(node == 0 ? 0.5 * s * (s - 1.0) : node == 1 ? 1.0 - s * s : 0.5 * s * (s + 1.0));
+}
+__host__ __device__ constexpr float q2_d(int point, int node) {
+    const double s = (point - 1) * kSqrt35;
+    return (float)(node == 0 ? s - 0.5 : node == 1 ? -2.0 * s : s + 0.5);
+}
+// Hexa_27 node (and Gauss point) number of the lattice position (a, b, c) in {0, 1, 2}^3.
+__host__ __device__ constexpr int q2_index(int a, int b, int c) {
+    constexpr int at[27] = {0, 8, 1, 11, 20, 9, 3, 10, 2, 12, 21, 13, 24, 26, 22, 15, 23, 14, 4, 16, 5, 19, 25, 17, 7, 18, 6};
+    return at[a + 3 * b + 9 * c];
+}
+
+// P3's weights, read by lane (E == 9 reads c_w9).
+__device__ const float g_w8f[11] = {ShapeConst<8>::w(0), ShapeConst<8>::w(1), ShapeConst<8>::w(2), ShapeConst<8>::w(3),
+                                    ShapeConst<8>::w(4), ShapeConst<8>::w(5), ShapeConst<8>::w(6), ShapeConst<8>::w(7),
+                                    ShapeConst<8>::w(8), ShapeConst<8>::w(9), ShapeConst<8>::w(10)};
+
+template <int E, int MAT>
+__global__ void __launch_bounds__(PointLanes<E>::kThreads, PointLanes<E>::kMinBlocks)
+k_vertex_points(const SceneDev* __restrict__ scenes, const VWork* __restrict__ work, int n_work, int mode, StepParams P,
+                double* red) {
+    constexpr int NE = ElemT<E>::NE, NQ = ElemT<E>::NQ, EW = EntryLayout<NE>::kWords;
+    constexpr int LP = PointLanes<E>::LP, PP = PointLanes<E>::PP, GW = 32 / LP, SLOTS = point_slots<E>();
+    constexpr int NI = (NE + LP - 1) / LP, NC = (9 + LP - 1) / LP;   // nodes and components per lane
+    __shared__ __align__(16) float s_dN[((NQ * NE * 3 + 3) / 4) * 4];
+    __shared__ __align__(16) float4 s_u[SLOTS][PointLanes<E>::kRow];
+    __shared__ float s_part[LP == 9 ? SLOTS : 1][LP * 9];
+    __shared__ float s_sum[SLOTS][9];
+    [[maybe_unused]] __shared__ float s_w[E == 8 ? NQ : 1];
+    __shared__ __align__(8) unsigned long long s_mbar;
+    const int lane = threadIdx.x & 31, g = lane / LP, j = lane - g * LP;
+    const bool on = g < GW;   // Q2: five lanes of a warp have no pair
+    const int slot = (threadIdx.x >> 5) * GW + (on ? g : 0);
+    const unsigned long long keep = policy_keep(), stream = policy_stream();
+    int scene, count, pair_base, n_pairs, r, rec, ids[NI];
+    int4 vertex;   // of this pair slot's vertex: node, first owner, owner count
+    auto fetch_pair = [&](const SceneDev& S, int p) {
+        const int* en = reinterpret_cast<const int*>(S.ent) + (size_t)(pair_base + p) * EW;
+        const bool has = on && p < n_pairs;
+#pragma unroll
+        for (int k = 0; k < NI; ++k) ids[k] = has && j + k * LP < NE ? ld_hint(en + j + k * LP, stream) & kIdMask : 0;
+        r = has ? ld_hint(en + NE, stream) : 0;
+        rec = has ? ld_hint(en + NE + 1, stream) : 0;
+    };
+    auto fetch = [&](int w) {   // static data of item w, up to its first round's node ids
+        const VWork wk = work[w];
+        scene = wk.scene; count = wk.count; pair_base = wk.pair_base; n_pairs = wk.n_pairs;
+        const SceneDev& S = scenes[scene];
+        vertex = on && slot < count ? __ldg(S.slots + wk.slot_begin + slot) : make_int4(0, 0, 0, 0);
+        fetch_pair(S, slot);
+    };
+    int w = blockIdx.x;
+    fetch(w);
+    [[maybe_unused]] float ny[3], dy[3], nz[3], dz[3];   // Q2: the lane's basis values along y and z
+    if constexpr (E == 9) {
+        const int b = j % 3, c = j / 3;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            ny[k] = b == 0 ? q2_n(0, k) : b == 1 ? q2_n(1, k) : q2_n(2, k);
+            dy[k] = b == 0 ? q2_d(0, k) : b == 1 ? q2_d(1, k) : q2_d(2, k);
+            nz[k] = c == 0 ? q2_n(0, k) : c == 1 ? q2_n(1, k) : q2_n(2, k);
+            dz[k] = c == 0 ? q2_d(0, k) : c == 1 ? q2_d(1, k) : q2_d(2, k);
+        }
+    }
+    [[maybe_unused]] int qs[PP];   // Q2: the lane's points (x = a) and their weights
+    [[maybe_unused]] float wts[PP];
+    if constexpr (E == 9) {
+#pragma unroll
+        for (int a = 0; a < PP; ++a) {
+            qs[a] = 0;
+#pragma unroll
+            for (int k = 0; k < 9; ++k) if (j == k) qs[a] = q2_index(a, k % 3, k / 3);
+            wts[a] = wq<E>(qs[a]);
+        }
+    } else {
+        if (threadIdx.x < NQ) s_w[threadIdx.x] = g_w8f[threadIdx.x];
+    }
+    stage_table(s_dN, gdN<E>(), NQ * NE * 3, &s_mbar, P.error);
+    pdl_wait();
+    while (true) {
+        const SceneDev& S = scenes[scene];
+        const bool mixed = S.precision != 0, affine = S.eq_stride == 1;
+        const bool active = on && slot < count && S.mask[vertex.x] != 0;
+        if (active && j == 0) {
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(S.u + vertex.x));
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(S.u_last + vertex.x));
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(S.y + vertex.x));
+        }
+        float sum[NC], cmp[NC];   // this lane's components of its slot's vertex
+#pragma unroll
+        for (int k = 0; k < NC; ++k) { sum[k] = 0.f; cmp[k] = 0.f; }
+        for (int base = 0; base < n_pairs; base += SLOTS) {
+            const bool has = on && base + slot < n_pairs;
+            if (base) fetch_pair(S, base + slot);
+            float acc[9];
+#pragma unroll
+            for (int k = 0; k < 9; ++k) acc[k] = 0.f;
+            if (has) {
+#pragma unroll
+                for (int k = 0; k < NI; ++k)
+                    if (j + k * LP < NE) s_u[slot][j + k * LP] = ld_hint(&S.u[ids[k]], keep);
+            }
+            const float4* R = affine ? S.rtab + 3 * (size_t)rec : S.eq + (size_t)rec * NQ * 3;
+            float4 A, B, C;
+            if (has && affine) { A = ld_hint(R, keep); B = ld_hint(R + 1, keep); C = ld_hint(R + 2, keep); }
+            __syncwarp();
+            if (has) {
+                // Q2: after z and y, per x-column of nodes: u_y u_z, u_y' u_z, u_y u_z' (value, d/dy, d/dz)
+                [[maybe_unused]] V3 cv[3], cy[3], cz[3];
+                if constexpr (E == 9) {
+#pragma unroll
+                    for (int a = 0; a < 3; ++a) {
+                        cv[a] = cy[a] = cz[a] = mk(0.f, 0.f, 0.f);
+#pragma unroll
+                        for (int b = 0; b < 3; ++b) {
+                            const V3 u0 = xyz(s_u[slot][q2_index(a, b, 0)]), u1 = xyz(s_u[slot][q2_index(a, b, 1)]),
+                                     u2 = xyz(s_u[slot][q2_index(a, b, 2)]);
+                            const V3 v = u0 * nz[0] + u1 * nz[1] + u2 * nz[2], d = u0 * dz[0] + u1 * dz[1] + u2 * dz[2];
+                            cv[a] = cv[a] + v * ny[b]; cy[a] = cy[a] + v * dy[b]; cz[a] = cz[a] + d * ny[b];
+                        }
+                    }
+                }
+                [[maybe_unused]] V3 un[E == 8 ? NE : 1];   // P3: the pair's nodes
+                if constexpr (E == 8) {
+#pragma unroll
+                    for (int i = 0; i < NE; ++i) un[i] = xyz(s_u[slot][i]);
+                }
+#pragma unroll (E == 9 ? PP : 1)
+                for (int a = 0; a < PP; ++a) {
+                    const int q = E == 9 ? qs[a] : j + a * LP;
+                    if (q >= NQ) continue;
+                    V3 J0 = mk(0, 0, 0), J1 = J0, J2 = J0;
+                    if constexpr (E == 9) {
+#pragma unroll
+                        for (int k = 0; k < 3; ++k) {
+                            J0 = J0 + cv[k] * q2_d(a, k); J1 = J1 + cy[k] * q2_n(a, k); J2 = J2 + cz[k] * q2_n(a, k);
+                        }
+                    } else {
+                        const float4* row = reinterpret_cast<const float4*>(&s_dN[q * NE * 3]);   // 15 x 16 B
+#pragma unroll
+                        for (int i = 0; i < NE / 4; ++i) {   // 4 nodes: 12 derivatives
+                            const float4 a0 = row[3 * i], a1 = row[3 * i + 1], a2 = row[3 * i + 2];
+                            const V3 u0 = un[4 * i], u1 = un[4 * i + 1], u2 = un[4 * i + 2], u3 = un[4 * i + 3];
+                            J0 = J0 + u0 * a0.x; J1 = J1 + u0 * a0.y; J2 = J2 + u0 * a0.z;
+                            J0 = J0 + u1 * a0.w; J1 = J1 + u1 * a1.x; J2 = J2 + u1 * a1.y;
+                            J0 = J0 + u2 * a1.z; J1 = J1 + u2 * a1.w; J2 = J2 + u2 * a2.x;
+                            J0 = J0 + u3 * a2.y; J1 = J1 + u3 * a2.z; J2 = J2 + u3 * a2.w;
+                        }
+                    }
+                    if (!affine) { A = ld_hint(R + 3 * q, stream); B = ld_hint(R + 3 * q + 1, stream); C = ld_hint(R + 3 * q + 2, stream); }
+                    const V3 m0 = mk(A.x, A.y, A.z), m1 = mk(A.w, B.x, B.y), m2 = mk(B.z, B.w, C.x);
+                    V3 F0 = J0 * m0.x + J1 * m0.y + J2 * m0.z;
+                    V3 F1 = J0 * m1.x + J1 * m1.y + J2 * m1.z;
+                    V3 F2 = J0 * m2.x + J1 * m2.y + J2 * m2.z;
+                    F0.x += 1.f; F1.y += 1.f; F2.z += 1.f;
+                    const float* dr = s_dN + (q * NE + r) * 3;
+                    const V3 dnr = mk(dr[0], dr[1], dr[2]);
+                    const V3 gr = mk(dot(m0, dnr), dot(m1, dnr), dot(m2, dnr));
+                    float t[9];
+                    material_terms<MAT>(F0, F1, F2, gr, C.z, C.w, C.y * (E == 9 ? wts[a] : s_w[q]), t);
+#pragma unroll
+                    for (int k = 0; k < 9; ++k) acc[k] += t[k];
+                }
+            }
+            // the pair's sums over its lanes into s_sum[slot]
+            if constexpr (LP == 9) {
+                if (on) {
+#pragma unroll
+                    for (int k = 0; k < 9; ++k) s_part[slot][j * 9 + k] = acc[k];
+                }
+                __syncwarp();
+                if (on) {
+                    float v = s_part[slot][j];
+#pragma unroll
+                    for (int k = 1; k < 9; ++k) v += s_part[slot][k * 9 + j];
+                    s_sum[slot][j] = v;
+                }
+            } else {
+#pragma unroll
+                for (int off = 1; off < LP; off <<= 1) {
+#pragma unroll
+                    for (int k = 0; k < 9; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], off);
+                }
+#pragma unroll
+                for (int k = 0; k < 9; ++k)
+                    if (k % LP == j) s_sum[slot][k] = acc[k];
+            }
+            __syncthreads();
+            // the vertex's pairs of this round, in owner order
+            if (active) {
+                const int p0 = max(vertex.y - pair_base, base), p1 = min(vertex.y - pair_base + vertex.z, base + SLOTS);
+                for (int p = p0; p < p1; ++p) {
+#pragma unroll
+                    for (int k = 0; k < NC; ++k) {
+                        const int comp = j + k * LP;
+                        if (comp >= 9) continue;
+                        const float v = s_sum[p - base][comp];
+                        if (mixed && comp < 3) kadd(sum[k], cmp[k], v);
+                        else sum[k] += v;
+                    }
+                }
+            }
+            __syncthreads();   // s_sum (and s_u) are written again by the next round
+        }
+        if (on) {
+#pragma unroll
+            for (int k = 0; k < NC; ++k)
+                if (j + k * LP < 9) s_sum[slot][j + k * LP] = sum[k] - cmp[k];
+        }
+        __syncwarp();
+        if (active && j == 0) {
+            float acc[9];
+#pragma unroll
+            for (int k = 0; k < 9; ++k) acc[k] = s_sum[slot][k];
+            vertex_epilogue(S, vertex.x, acc, mode, P, red);
+        }
+        w += gridDim.x;
+        if (w >= n_work) break;
+        fetch(w);
+    }
+    pdl_trigger();
+}
 
 // ------------------------------------------------------------------------ colour kernel
 // mode 0: VBD solve; mode 1: VBD residual (r into u_new, |r| reductions).
@@ -800,6 +1055,24 @@ __global__ void __launch_bounds__(kBlock, LaneMinBlocks<E>::value) k_vertex(cons
 // ------------------------------------------------------------------------ node kernels
 constexpr int kNodeChunk = 256;
 
+// Predictor of a VBD sub-step for node i (kernel_integration, GPU_VBD.cu:6-18): pending, the
+// initial velocity is the implicit velocity (u - u_last)/dt of the scene's first sub-step.
+__device__ __forceinline__ void vbd_predict(const SceneDev& S, int i, bool pending, bool chebyshev, float dt, float inv_dt) {
+    float4 u = S.u[i], ul = S.u_last[i];
+    if (pending) {
+        const float4 v = S.v[i];
+        ul = make_float4(u.x - v.x * dt, u.y - v.y * dt, u.z - v.z * dt, ul.w);
+    }
+    if (chebyshev) S.prev1[i] = u;
+    float4 y = S.y[i];
+    y.x = u.x + ((u.x - ul.x) * inv_dt + S.gx * dt) * dt;
+    y.y = u.y + ((u.y - ul.y) * inv_dt + S.gy * dt) * dt;
+    y.z = u.z + ((u.z - ul.z) * inv_dt + S.gz * dt) * dt;
+    S.y[i] = y;
+    S.u_last[i] = u;
+    S.u[i] = make_float4(y.x, y.y, y.z, u.w);
+}
+
 // Sub-step predictor.  kind 0: VBD (kernel_integration, GPU_VBD.cu:6-18) with the
 // Chebyshev history seed; kind 1: semi-implicit Euler (kenerl_semi_exicit_integration,
 // GPU_Integrator.cu:27-34), force taken from u_new for the explicit solver when use_force.
@@ -813,22 +1086,10 @@ __global__ void k_predict(const SceneDev* __restrict__ scenes, const NWork* __re
     const SceneDev& S = scenes[wk.scene];
     const int i = wk.begin + threadIdx.x;
     const float dt = P.dt;
-    float4 u = S.u[i], ul = S.u_last[i];
     if (kind == 0) {
-        if (P.pending_v0 && P.pending_v0[wk.scene]) {   // initial velocity as the implicit velocity (u - u_last)/dt
-            const float4 v = S.v[i];
-            ul = make_float4(u.x - v.x * dt, u.y - v.y * dt, u.z - v.z * dt, ul.w);
-        }
-        if (chebyshev) S.prev1[i] = u;
-        float4 y = S.y[i];
-        y.x = u.x + ((u.x - ul.x) * P.inv_dt + S.gx * dt) * dt;
-        y.y = u.y + ((u.y - ul.y) * P.inv_dt + S.gy * dt) * dt;
-        y.z = u.z + ((u.z - ul.z) * P.inv_dt + S.gz * dt) * dt;
-        S.y[i] = y;
-        S.u_last[i] = u;
-        S.u[i] = make_float4(y.x, y.y, y.z, u.w);
+        vbd_predict(S, i, P.pending_v0 && P.pending_v0[wk.scene], chebyshev, dt, P.inv_dt);
     } else {
-        float4 v = S.v[i];
+        float4 u = S.u[i], v = S.v[i];
         const float w = 1.f / S.y[i].w;
         float fx = 0.f, fy = 0.f, fz = 0.f;
         if (use_force) { const float4 f = S.u_new[i]; fx = f.x; fy = f.y; fz = f.z; }
@@ -841,6 +1102,15 @@ __global__ void k_predict(const SceneDev* __restrict__ scenes, const NWork* __re
     }
 }
 
+// Velocity of node i at the end of a VBD sub-step (kernel_velocity_update, GPU_VBD.cu:20-25), and
+// the one check per node that flags a scene whose state blew up.
+__device__ __forceinline__ void vbd_velocity(const SceneDev& S, int i, float dt) {
+    const float4 u = S.u[i], ul = S.u_last[i];
+    const float4 v = make_float4((u.x - ul.x) / dt, (u.y - ul.y) / dt, (u.z - ul.z) / dt, 0.f);
+    S.v[i] = v;
+    if (!isfinite(u.x + u.y + u.z + v.x + v.y + v.z)) atomicOr(S.status, kStatusNonFinite);
+}
+
 // kernel_velocity_update (GPU_VBD.cu:20-25); with global damping for XPBD (GPU_PBD.cu:8-18).
 __global__ void k_velocity(const SceneDev* __restrict__ scenes, const NWork* __restrict__ work, int n_work, int pbd,
                            StepParams P) {
@@ -850,9 +1120,10 @@ __global__ void k_velocity(const SceneDev* __restrict__ scenes, const NWork* __r
     if (threadIdx.x >= wk.count) return;
     const SceneDev& S = scenes[wk.scene];
     const int i = wk.begin + threadIdx.x;
+    if (!pbd) { vbd_velocity(S, i, P.dt); return; }
     const float4 u = S.u[i], ul = S.u_last[i];
     float4 v = make_float4((u.x - ul.x) / P.dt, (u.y - ul.y) / P.dt, (u.z - ul.z) / P.dt, 0.f);
-    if (pbd) {
+    {
         const float nv = sqrtf(v.x * v.x + v.y * v.y + v.z * v.z);
         if (nv > 1e-7f) {
             const float coef = S.global_damping * P.dt / S.y[i].w;
@@ -866,21 +1137,22 @@ __global__ void k_velocity(const SceneDev* __restrict__ scenes, const NWork* __r
 }
 
 // Chebyshev semi-iterative acceleration (kernel_chebychev_acceleration, GPU_VBD.cu:27-36).
+__device__ __forceinline__ void chebyshev_node(const SceneDev& S, int i, int iteration, float omega) {
+    float4 u = S.u[i];
+    const float4 p2 = S.prev2[i];
+    if (iteration >= 2) {
+        u.x = p2.x + omega * (u.x - p2.x); u.y = p2.y + omega * (u.y - p2.y); u.z = p2.z + omega * (u.z - p2.z);
+        S.u[i] = u;
+    }
+    S.prev2[i] = S.prev1[i];
+    S.prev1[i] = u;
+}
 __global__ void k_chebyshev(const SceneDev* __restrict__ scenes, const NWork* __restrict__ work, int n_work, StepParams P) {
     pdl_trigger();
     pdl_wait();
     const NWork wk = work[blockIdx.x];
     if (threadIdx.x >= wk.count) return;
-    const SceneDev& S = scenes[wk.scene];
-    const int i = wk.begin + threadIdx.x;
-    float4 u = S.u[i];
-    const float4 p2 = S.prev2[i];
-    if (P.iteration >= 2) {
-        u.x = p2.x + P.omega * (u.x - p2.x); u.y = p2.y + P.omega * (u.y - p2.y); u.z = p2.z + P.omega * (u.z - p2.z);
-        S.u[i] = u;
-    }
-    S.prev2[i] = S.prev1[i];
-    S.prev1[i] = u;
+    chebyshev_node(scenes[wk.scene], wk.begin + threadIdx.x, P.iteration, P.omega);
 }
 
 // Fixed nodes (kernel_constraint_fix, GPU_Constraint.cu:8-20) then, if enabled, the box
@@ -1755,7 +2027,7 @@ void launch_pdl(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem
     cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
-template <class K> int persistent_grid(K kernel, int n_work, size_t smem = 0) {
+template <class K> int persistent_grid(K kernel, int block, int n_work, size_t smem = 0) {
     static int sms = 0;
     if (!sms) {
         int dev = 0;
@@ -1763,7 +2035,7 @@ template <class K> int persistent_grid(K kernel, int n_work, size_t smem = 0) {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     }
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kBlock, smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, smem);
     if (per_sm < 1) per_sm = 1;
     const int g = sms * per_sm;
     return n_work < g ? n_work : g;
@@ -1771,43 +2043,55 @@ template <class K> int persistent_grid(K kernel, int n_work, size_t smem = 0) {
 
 // Persistent grid size (SMs x resident blocks) of each vertex-kernel instantiation,
 // computed once outside any stream capture by prepare_vertex.
-template <int E, int MAT, bool PACKED> int& grid_cap() {
+template <int E, int MAT, int FORM> int& grid_cap() {
     static int cap = 0;
     return cap;
 }
 
+// Forms of an element's packed mapping: one lane per pair (not Q2), point lanes (P3, Q2).
+template <int E> constexpr bool kPairLanes = E != 9;
+template <int E> constexpr bool kPointLanes = E == 8 || E == 9;
+
 template <int E, int MAT>
-void vertex_dispatch(const SceneDev* scenes, const VWork* work, int n_work, int tpv, int mode, const StepParams& P,
+void vertex_dispatch(const SceneDev* scenes, const VWork* work, int n_work, int form, int mode, const StepParams& P,
                      double* red, cudaStream_t st) {
     if (mode < 0) {   // preparation call: fill the caches only
-        if (grid_cap<E, MAT, false>() <= 0) grid_cap<E, MAT, false>() = persistent_grid(k_vertex<E, MAT>, 1 << 30);
-        if (grid_cap<E, MAT, true>() <= 0) {
-            cudaFuncSetAttribute(k_vertex_packed<E, MAT>, cudaFuncAttributeMaxDynamicSharedMemorySize, packed_smem_bytes<E>());
-            grid_cap<E, MAT, true>() = persistent_grid(k_vertex_packed<E, MAT>, 1 << 30, packed_smem_bytes<E>());
-        }
+        if (grid_cap<E, MAT, 1>() <= 0) grid_cap<E, MAT, 1>() = persistent_grid(k_vertex<E, MAT>, kBlock, 1 << 30);
+        if constexpr (kPairLanes<E>)
+            if (grid_cap<E, MAT, 0>() <= 0) {
+                cudaFuncSetAttribute(k_vertex_packed<E, MAT>, cudaFuncAttributeMaxDynamicSharedMemorySize, packed_smem_bytes<E>());
+                grid_cap<E, MAT, 0>() = persistent_grid(k_vertex_packed<E, MAT>, kBlock, 1 << 30, packed_smem_bytes<E>());
+            }
+        if constexpr (kPointLanes<E>)
+            if (grid_cap<E, MAT, -1>() <= 0)
+                grid_cap<E, MAT, -1>() = persistent_grid(k_vertex_points<E, MAT>, PointLanes<E>::kThreads, 1 << 30);
         return;
     }
-    if (tpv == 0) {
-        int cap = grid_cap<E, MAT, true>();
-        if (cap <= 0) cap = 148 * 4;
-        const int blocks = (n_work + kBlock / 32 - 1) / (kBlock / 32);
-        launch_pdl(k_vertex_packed<E, MAT>, blocks < cap ? blocks : cap, kBlock, packed_smem_bytes<E>(), st, scenes, work, n_work, mode, P, red);
-        return;
+    auto capped = [&](int cap, int blocks, int per_sm) {
+        if (cap <= 0) cap = 148 * per_sm;
+        return blocks < cap ? blocks : cap;
+    };
+    if (form > 0) {
+        launch_pdl(k_vertex<E, MAT>, capped(grid_cap<E, MAT, 1>(), n_work, 4), kBlock, 0, st, scenes, work, n_work, mode, P, red);
+    } else if (form == 0) {
+        if constexpr (kPairLanes<E>)
+            launch_pdl(k_vertex_packed<E, MAT>, capped(grid_cap<E, MAT, 0>(), (n_work + kBlock / 32 - 1) / (kBlock / 32), 4), kBlock,
+                       packed_smem_bytes<E>(), st, scenes, work, n_work, mode, P, red);
+    } else {
+        if constexpr (kPointLanes<E>)
+            launch_pdl(k_vertex_points<E, MAT>, capped(grid_cap<E, MAT, -1>(), n_work, 1), PointLanes<E>::kThreads, 0, st, scenes, work,
+                       n_work, mode, P, red);
     }
-    int cap = grid_cap<E, MAT, false>();
-    if (cap <= 0) cap = 148 * 4;
-    const int grid = n_work < cap ? n_work : cap;
-    launch_pdl(k_vertex<E, MAT>, grid, kBlock, 0, st, scenes, work, n_work, mode, P, red);
 }
 
 template <int E>
-void vertex_mat(int mat, const SceneDev* scenes, const VWork* work, int n_work, int tpv, int mode, const StepParams& P,
+void vertex_mat(int mat, const SceneDev* scenes, const VWork* work, int n_work, int form, int mode, const StepParams& P,
                 double* red, cudaStream_t st) {
     switch (mat) {
-        case 0: vertex_dispatch<E, 0>(scenes, work, n_work, tpv, mode, P, red, st); break;
-        case 1: vertex_dispatch<E, 1>(scenes, work, n_work, tpv, mode, P, red, st); break;
-        case 2: vertex_dispatch<E, 2>(scenes, work, n_work, tpv, mode, P, red, st); break;
-        default: vertex_dispatch<E, 3>(scenes, work, n_work, tpv, mode, P, red, st); break;
+        case 0: vertex_dispatch<E, 0>(scenes, work, n_work, form, mode, P, red, st); break;
+        case 1: vertex_dispatch<E, 1>(scenes, work, n_work, form, mode, P, red, st); break;
+        case 2: vertex_dispatch<E, 2>(scenes, work, n_work, form, mode, P, red, st); break;
+        default: vertex_dispatch<E, 3>(scenes, work, n_work, form, mode, P, red, st); break;
     }
 }
 
@@ -1924,15 +2208,15 @@ void prepare_vertex(int element, int material) {
     launch_vertex(element, material, nullptr, nullptr, 1, 1, -1, P, nullptr, nullptr);
 }
 
-void launch_vertex(int element, int material, const SceneDev* scenes, const VWork* work, int n_work, int tpv, int mode,
+void launch_vertex(int element, int material, const SceneDev* scenes, const VWork* work, int n_work, int form, int mode,
                    const StepParams& P, double* red, cudaStream_t st) {
     if (n_work <= 0) return;
     switch (element) {
-        case 3: vertex_mat<3>(material, scenes, work, n_work, tpv, mode, P, red, st); break;
-        case 6: vertex_mat<6>(material, scenes, work, n_work, tpv, mode, P, red, st); break;
-        case 7: vertex_mat<7>(material, scenes, work, n_work, tpv, mode, P, red, st); break;
-        case 8: vertex_mat<8>(material, scenes, work, n_work, tpv, mode, P, red, st); break;
-        case 9: vertex_mat<9>(material, scenes, work, n_work, tpv, mode, P, red, st); break;
+        case 3: vertex_mat<3>(material, scenes, work, n_work, form, mode, P, red, st); break;
+        case 6: vertex_mat<6>(material, scenes, work, n_work, form, mode, P, red, st); break;
+        case 7: vertex_mat<7>(material, scenes, work, n_work, form, mode, P, red, st); break;
+        case 8: vertex_mat<8>(material, scenes, work, n_work, form, mode, P, red, st); break;
+        case 9: vertex_mat<9>(material, scenes, work, n_work, form, mode, P, red, st); break;
     }
 }
 
@@ -2023,6 +2307,8 @@ void launch_explicit_force(int element, int material, const SceneDev* scene, int
         launch_pdl(k_explicit_gather, n_slots, kNodeChunk, 0, st, scene, slots, (const float4*)contrib,
                    element == 3 ? 4 : element == 6 ? 8 : element == 7 ? 10 : element == 8 ? 20 : 27, P);
 }
+
+int point_item_pairs(int element) { return element == 8 ? point_slots<8>() : point_slots<9>(); }
 
 int xpbd_elements_per_block(int element) {
     switch (element) {

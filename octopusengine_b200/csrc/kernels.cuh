@@ -11,8 +11,9 @@ cudaError_t upload_shape_tables_fp64(int element, const double* dN, int n, const
 // Caches the persistent grid size of the vertex kernel for (element, material); call
 // outside stream capture.
 void prepare_vertex(int element, int material);
+// form > 0: lane-group items, 0: packed items, one lane per pair, -1: point-lane items (P3, Q2).
 // mode 0: VBD solve, 1: VBD residual (red[0] += |r|, red[1] = max |r|)
-void launch_vertex(int element, int material, const SceneDev* scenes, const VWork* work, int n_work, int tpv, int mode,
+void launch_vertex(int element, int material, const SceneDev* scenes, const VWork* work, int n_work, int form, int mode,
                    const StepParams& P, double* red, cudaStream_t st);
 void launch_commit(const SceneDev* scenes, const VWork* work, int n_work, cudaStream_t st);
 // Explicit sub-step without the constraints: the element-centric force pass (per-(element,
@@ -48,6 +49,8 @@ void launch_effect(const SceneDev* scene, const NWork* work, int n_work, int slo
 void launch_xpbd(int element, int material, bool raw, const SceneDev* scenes, const XWork* work, int n_work,
                  const StepParams& P, cudaStream_t st);
 int xpbd_elements_per_block(int element);
+// (vertex, owner) pairs that one work item of the point lanes holds
+int point_item_pairs(int element);
 // Per-element diagnostics of GPU_FEM (kind 0 stress, 1 volume, 2 volume change, 3 inverted,
 // 4 stress with the reference kernel's accumulated Jx).
 void launch_element_diag(int element, int material, const SceneDev* scenes, int scene, int n_elements, int kind, float* out,

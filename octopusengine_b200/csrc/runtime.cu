@@ -170,6 +170,7 @@ struct oct_scene {
     int* d_status = nullptr;        // SceneDev::status of the scene's own steps
     VWork* d_vwork = nullptr;
     std::vector<int> vwork_off;     // per colour: [vwork_off[c], vwork_off[c+1])
+    std::vector<int> form;          // per colour: launch_form
     NWork* d_nwork = nullptr;
     int n_nwork = 0;
     NWork* d_fwork = nullptr;
@@ -212,6 +213,7 @@ struct oct_batch {
         int element, material, tpv;     // XPBD: tpv holds the raw (V1/V2) update flag
         bool in_place;
         std::vector<int> off;   // per colour, into the group's part of d_vwork (XPBD: d_xwork)
+        std::vector<int> form;  // per colour: launch_form (VBD)
         int base = 0;
         cudaStream_t stream = nullptr;
         cudaEvent_t done = nullptr;
@@ -262,8 +264,10 @@ constexpr int kOwnersPerLane = 8;
 // measured_tpv, used when the description leaves the lanes at 0
 int measured_tpv(int element);
 
-// Lanes of one scene's colour.  least: as above.  width: with the default mapping, the power of
-// two nearest the colour's owners per vertex (about one owner per lane); else least.
+// Lanes of one scene's colour.  least: as above.  width: with the default mapping, lanes for the
+// owners of the colour's vertex of most owners, one each (P1: three, whose one point is a small
+// part of what a vertex costs: an 81-node sub-step in one block 146 us with 8 lanes, 260 us with
+// 32); else least.
 struct ColourLanes {
     int least = 1, width = 1;
     int at(int div) const { return std::max(least, width / div); }
@@ -276,7 +280,8 @@ ColourLanes colour_lanes(int element, int tpv, int begin, int end, const std::ve
     while (l.least < 32 && pairs > (int64_t)kOwnersPerLane * l.least * n) l.least <<= 1;
     l.width = l.least;
     if (tpv != measured_tpv(element)) return l;
-    while (l.width < 32 && 2 * pairs >= 3 * (int64_t)l.width * n) l.width <<= 1;
+    const int each = element == kTetra ? 3 : 1;   // the vertices are in the order of decreasing owner count
+    while (l.width < 32 && each * l.width < own_off[begin + 1] - own_off[begin]) l.width <<= 1;
     return l;
 }
 
@@ -296,24 +301,37 @@ int lane_div(int64_t full) {
     return div;
 }
 
+// How a colour launch of `pairs` (vertex, owner) pairs is run: tpv > 0 lane groups; else the
+// packed mapping, 0 one lane per pair, -1 point lanes (k_vertex_points).  Q2 always takes point
+// lanes; P3 while its items are about one wave (frame of 20 sweeps, point lanes / one lane per
+// pair: 1,000 nodes 2.7 / 3.3 ms, 50,653 nodes 3.4 / 4.0, 493,039 nodes 23 / 13).
+int launch_form(int element, int tpv, int64_t pairs) {
+    if (tpv > 0) return tpv;
+    constexpr int64_t kWavePairs = 12000;
+    return element == kHexa27 || (element == kTetra20 && pairs <= kWavePairs) ? -1 : 0;
+}
+
 // Split [begin, end) slots into work items for one scene: block-sized items of 128 / t slots
-// (l, div as above), or (tpv == 0) warp items packing whole vertices up to 32 (vertex, owner)
-// pairs and at most 31 slots.
-void append_vwork(std::vector<VWork>& out, int scene, int begin, int end, int tpv, ColourLanes l, int div,
+// (l, div as above), or packed items of whole vertices up to the kernel's (vertex, owner) pairs
+// per item; a vertex of more pairs than that (point lanes only) is an item by itself.
+void append_vwork(std::vector<VWork>& out, int scene, int element, int begin, int end, int form, ColourLanes l, int div,
                   const std::vector<int32_t>& own_off) {
-    if (tpv > 0) {
+    if (form > 0) {
         const int t = l.at(div), vpb = kBlockThreads / t;
         for (int s = begin; s < end; s += vpb)
             out.push_back({scene, s, std::min(vpb, end - s), t, 0, 0u, 0, 0});
         return;
     }
+    const int most = form < 0 ? point_item_pairs(element) : 32, most_n = form < 0 ? most : 31;
     int s = begin;
     while (s < end) {
         int pairs = 0, n = 0;
         unsigned heads = 0;
-        while (s + n < end && n < 31 && pairs + (own_off[s + n + 1] - own_off[s + n]) <= 32) {
-            heads |= 1u << pairs;
-            pairs += own_off[s + n + 1] - own_off[s + n];
+        while (s + n < end && n < most_n) {
+            const int v = own_off[s + n + 1] - own_off[s + n];
+            if (n && pairs + v > most) break;
+            if (pairs < 32) heads |= 1u << pairs;   // read by the one-lane-per-pair kernel
+            pairs += v;
             ++n;
         }
         out.push_back({scene, s, n, 0, own_off[s], heads, pairs, 0});
@@ -368,10 +386,12 @@ oct_status check_error_word(oct_ctx* c) {
 oct_status build_vertex_work(oct_scene* s) {
     std::vector<VWork> vw;
     s->vwork_off.assign(1, 0);
+    s->form.clear();
     for (int k = 0; k + 1 < (int)s->color_off.size(); ++k) {
         const int begin = s->color_off[k], end = s->color_off[k + 1];
         const ColourLanes l = colour_lanes(s->element, s->tpv, begin, end, s->own_off);
-        append_vwork(vw, 0, begin, end, s->tpv, l, lane_div((int64_t)l.width * (end - begin)), s->own_off);
+        s->form.push_back(launch_form(s->element, s->tpv, (int64_t)s->own_off[end] - s->own_off[begin]));
+        append_vwork(vw, 0, s->element, begin, end, s->form[k], l, lane_div((int64_t)l.width * (end - begin)), s->own_off);
         s->vwork_off.push_back((int)vw.size());
     }
     return upload(s->ctx, s->mem, s->d_vwork, vw);
@@ -731,7 +751,7 @@ oct_status build_scene(oct_ctx* c, const oct_scene_desc* d, oct_scene* s) {
     h.u = u; h.u_last = ul; h.y = y; h.v = v; h.u_new = un; h.prev1 = p1; h.prev2 = p2; h.mask = maskd; h.X = Xd;
     h.topo = topod; h.eq = eqd; h.vids = vidsd; h.own_off = offd; h.owners = ownd; h.fixed = fixd;
     h.fixed_group = fgd; h.fix = s->d_fix;
-    if (d->solver == OCT_SOLVER_EXPLICIT && s->n_fixed) {   // the explicit update applies the fixation itself
+    if (d->solver != OCT_SOLVER_XPBD && s->n_fixed) {   // for the updates that apply the fixation node by node
         std::vector<int32_t> fix_of(N, -1);
         for (int k = 0; k < s->n_fixed; ++k) fix_of[s->fixed[k]] = s->fixed_group[k];
         int* fod;
@@ -907,12 +927,14 @@ void vbd_substep(oct_scene* s, float dt) {
     P.pending_v0 = s->d_pending;
     P.in_place = s->in_place ? 1 : 0;
     const bool cheb = s->rho > 0.f && s->rho > 1.17549435e-38f * 1e6f;
-    launch_predict(s->d_scene, s->d_nwork, s->n_nwork, 0, 0, cheb ? 1 : 0, P, st);
-    c->launches++;
-    if (s->pending_host) {
+    auto consumed = [&] {   // the pending initial velocity, by the predictor
+        if (!s->pending_host) return;
         cudaMemsetAsync(s->d_pending, 0, sizeof(int), st);
         s->pending_host = 0;
-    }
+    };
+    launch_predict(s->d_scene, s->d_nwork, s->n_nwork, 0, 0, cheb ? 1 : 0, P, st);
+    c->launches++;
+    consumed();
     std::vector<int> order(s->n_colors);
     float omega = 1.f;
     for (int j = 0; j < s->iterations; ++j) {
@@ -932,7 +954,7 @@ void vbd_substep(oct_scene* s, float dt) {
                 PL.pending_v0 = nullptr;
                 for (int k = 0; k < L->n_colors; ++k) {
                     const int b = L->vwork_off[k], n = L->vwork_off[k + 1] - b;
-                    launch_vertex(L->element, L->material, L->d_scene, L->d_vwork + b, n, L->tpv, 0, PL, nullptr, st);
+                    launch_vertex(L->element, L->material, L->d_scene, L->d_vwork + b, n, L->form[k], 0, PL, nullptr, st);
                     if (!L->in_place) launch_commit(L->d_scene, L->d_vwork + b, n, st);
                     c->launches += L->in_place ? 1 : 2;
                 }
@@ -950,7 +972,7 @@ void vbd_substep(oct_scene* s, float dt) {
         Range sweep("colour_sweep");
         for (int k : order) {
             const int b = s->vwork_off[k], n = s->vwork_off[k + 1] - b;
-            launch_vertex(s->element, s->material, s->d_scene, s->d_vwork + b, n, s->tpv, 0, P, nullptr, st);
+            launch_vertex(s->element, s->material, s->d_scene, s->d_vwork + b, n, s->form[k], 0, P, nullptr, st);
             c->launches++;
             if (!s->in_place) { launch_commit(s->d_scene, s->d_vwork + b, n, st); c->launches++; }
         }
@@ -1524,7 +1546,7 @@ oct_status oct_scene_vertex_residuals(oct_scene* s, float dt, float* out) {
     OCT_CUDA(c, cudaMemsetAsync(s->h.u_new, 0, sizeof(float4) * s->n_nodes, c->stream));
     for (int k = 0; k < s->n_colors; ++k) {
         const int b = s->vwork_off[k], n = s->vwork_off[k + 1] - b;
-        launch_vertex(s->element, s->material, s->d_scene, s->d_vwork + b, n, s->tpv, 1, P, s->d_red, c->stream);
+        launch_vertex(s->element, s->material, s->d_scene, s->d_vwork + b, n, s->form[k], 1, P, s->d_red, c->stream);
     }
     OCT_CUDA(c, cudaGetLastError());
     oct_status st = read_nodes(s, s->h.u_new, out, false);
@@ -1540,7 +1562,7 @@ oct_status oct_scene_residual(oct_scene* s, float dt, double out[2]) {
     OCT_CUDA(c, cudaMemsetAsync(s->d_red, 0, 4 * sizeof(double), c->stream));
     for (int k = 0; k < s->n_colors; ++k) {
         const int b = s->vwork_off[k], n = s->vwork_off[k + 1] - b;
-        launch_vertex(s->element, s->material, s->d_scene, s->d_vwork + b, n, s->tpv, 1, P, s->d_red, c->stream);
+        launch_vertex(s->element, s->material, s->d_scene, s->d_vwork + b, n, s->form[k], 1, P, s->d_red, c->stream);
     }
     OCT_CUDA(c, cudaMemcpyAsync(out, s->d_red, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     OCT_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -1683,17 +1705,22 @@ oct_status oct_batch_create(oct_ctx* c, oct_scene* const* scenes, int n, oct_bat
         for (int i : members[g]) cw.resize(std::max(cw.size(), (size_t)scenes[i]->n_colors));
         for (int k = 0; k < (int)cw.size(); ++k) {
             std::vector<ColourLanes> l;
-            int64_t full = 0;
+            int64_t full = 0, pairs = 0;
             for (int i : members[g]) {
                 const oct_scene* s = scenes[i];
                 const bool has = k < s->n_colors;
                 l.push_back(has ? colour_lanes(s->element, s->tpv, s->color_off[k], s->color_off[k + 1], s->own_off) : ColourLanes());
-                if (has) full += (int64_t)l.back().width * (s->color_off[k + 1] - s->color_off[k]);
+                if (!has) continue;
+                full += (int64_t)l.back().width * (s->color_off[k + 1] - s->color_off[k]);
+                pairs += s->own_off[s->color_off[k + 1]] - s->own_off[s->color_off[k]];
             }
+            auto& form = b->groups[g].form;
+            form.push_back(launch_form(b->groups[g].element, b->groups[g].tpv, pairs));
             for (size_t m = 0; m < members[g].size(); ++m) {
                 const oct_scene* s = scenes[members[g][m]];
                 if (k < s->n_colors)
-                    append_vwork(cw[k], members[g][m], s->color_off[k], s->color_off[k + 1], s->tpv, l[m], lane_div(full), s->own_off);
+                    append_vwork(cw[k], members[g][m], s->element, s->color_off[k], s->color_off[k + 1], form[k], l[m],
+                                 lane_div(full), s->own_off);
             }
         }
     }
@@ -1784,7 +1811,7 @@ void batch_substep(oct_batch* b, float dt) {
             for (size_t k = 0; k + 1 < g.off.size(); ++k) {
                 const VWork* w = b->d_vwork + g.base + g.off[k];
                 const int n = g.off[k + 1] - g.off[k];
-                launch_vertex(g.element, g.material, b->d_scenes, w, n, g.tpv, 0, Pg, nullptr, g.stream);
+                launch_vertex(g.element, g.material, b->d_scenes, w, n, g.form[k], 0, Pg, nullptr, g.stream);
                 if (!g.in_place) launch_commit(b->d_scenes, w, n, g.stream);
             }
             cudaEventRecord(g.done, g.stream);
@@ -1916,7 +1943,7 @@ oct_status oct_batch_time_group(oct_batch* b, int g, int sweeps, float dt, float
         for (size_t k = 0; k + 1 < G.off.size(); ++k) {
             const VWork* w = b->d_vwork + G.base + G.off[k];
             const int n = G.off[k + 1] - G.off[k];
-            launch_vertex(G.element, G.material, b->d_scenes, w, n, G.tpv, 0, P, nullptr, c->stream);
+            launch_vertex(G.element, G.material, b->d_scenes, w, n, G.form[k], 0, P, nullptr, c->stream);
             if (!G.in_place) launch_commit(b->d_scenes, w, n, c->stream);
             c->launches += G.in_place ? 1 : 2;
         }
@@ -1964,7 +1991,7 @@ static oct_status time_batch_sweeps(oct_batch* b, int sweeps, float dt, float* m
         for (const auto& G : b->groups)
             for (size_t k = 0; k + 1 < G.off.size(); ++k) {
                 const int n = G.off[k + 1] - G.off[k];
-                launch_vertex(G.element, G.material, b->d_scenes, b->d_vwork + G.base + G.off[k], n, G.tpv, 0, P, nullptr,
+                launch_vertex(G.element, G.material, b->d_scenes, b->d_vwork + G.base + G.off[k], n, G.form[k], 0, P, nullptr,
                               c->stream);
             }
     OCT_CUDA(c, cudaEventRecord(c->ev1, c->stream));
