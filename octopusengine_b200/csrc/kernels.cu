@@ -1194,6 +1194,157 @@ __global__ void k_constraints(const SceneDev* __restrict__ scenes, const NWork* 
     }
 }
 
+// ------------------------------------------------------------------------ VBD sub-step
+// One VBD sub-step of one scene in one cooperative launch: predictor, iterations x (colour sweeps,
+// fixation in the first, Chebyshev), velocity update, with a grid barrier where the launch path
+// has a kernel boundary.  At a kernel boundary a colour of a few thousand vertices pays the
+// drain, the flush, the launch and then its static loads one after the other (3.3 us for a colour
+// of 20 vertices, 4 us for one of 360); here a block has its next colour's work item, slot and
+// owner entry in flight while it waits for the others.  The colours' work items, lanes and
+// arithmetic are those of k_vertex, so the results are the same bits.
+//
+// Blocks of 512 threads, at most one per SM, are four sub-blocks of 128, each taking items of the
+// colour in turn (first one per SM).  A scene whose colours fit a few items runs in one block, and
+// its barrier is __syncthreads.  The SceneDev is copied to shared memory: the barrier's acquire
+// empties L1.
+constexpr int kSubBlocks = 4;
+
+// Barrier over the grid: bar[0] counts arrivals.  The wait has an iteration limit; a block that
+// gives up records the time-out and returns false, and so do the others that it leaves waiting.
+struct GridBarrier {
+    unsigned* bar;
+    unsigned target;
+    bool alive;
+    __device__ __forceinline__ void arrive() {
+        __syncthreads();
+        if (gridDim.x == 1) return;
+        target += gridDim.x;
+        if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+    }
+    __device__ __forceinline__ bool wait(int* error) {
+        if (gridDim.x > 1 && threadIdx.x == 0) {
+            unsigned seen = 0;
+            int it = 0;
+            do {
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
+            } while ((int)(seen - target) < 0 && ++it < (1 << 20));
+            if ((int)(seen - target) < 0) { atomicOr(error, 1); alive = false; }
+        }
+        return !__syncthreads_or(threadIdx.x == 0 && !alive);
+    }
+};
+
+template <int E, int MAT>
+__global__ void __launch_bounds__(kSubBlocks * kBlock, 1)
+k_vbd_substep(const SceneDev* __restrict__ scene, const VWork* __restrict__ work, const int* __restrict__ colour_off,
+              int n_colours, int iterations, float rho, unsigned* bar, StepParams P) {
+    constexpr int NE = ElemT<E>::NE, NQ = ElemT<E>::NQ;
+    constexpr int EW = EntryLayout<NE>::kWords;
+    __shared__ __align__(128) float s_dN[((NQ * NE * 3 + 3) / 4) * 4];
+    __shared__ __align__(16) SceneDev s_scene;
+    for (int i = threadIdx.x; i < (int)(sizeof(SceneDev) / 4); i += blockDim.x)
+        reinterpret_cast<int*>(&s_scene)[i] = reinterpret_cast<const int*>(scene)[i];
+    for (int i = threadIdx.x; i < NQ * NE * 3; i += blockDim.x) s_dN[i] = gdN<E>()[i];
+    __syncthreads();
+    const SceneDev& S = s_scene;
+    const unsigned long long stream = policy_stream();
+    const int lane = threadIdx.x & 31, tid = threadIdx.x & (kBlock - 1);
+    const int first = (threadIdx.x / kBlock) * gridDim.x + blockIdx.x, step = gridDim.x * kSubBlocks;
+    const int node0 = blockIdx.x * blockDim.x + threadIdx.x, nodes = gridDim.x * blockDim.x;
+    const bool mixed = S.precision != 0, cheb = rho > 0.f;
+    int t = 1, glane = 0, o = 0, oe = 0, vid = -1;   // this lane's part of its next item
+    float4 nxt[EW / 4];
+    auto fetch = [&](int w, int end) {
+        vid = -1; o = oe = 0; t = 1; glane = 0;
+        if (w >= end) return;
+        const int4 wk = __ldg(reinterpret_cast<const int4*>(work + w));   // scene, slot_begin, count, lanes
+        t = wk.w;
+        glane = lane & (t - 1);
+        const int group = tid >> (__ffs(t) - 1);
+        if (group >= wk.z) return;
+        const int4 sl = __ldg(S.slots + wk.y + group);
+        vid = sl.x;
+        o = sl.y + glane;
+        oe = sl.y + sl.z;
+        if (o < oe) {
+#pragma unroll
+            for (int j = 0; j < EW / 4; ++j) nxt[j] = ld_hint(S.ent + (size_t)o * (EW / 4) + j, stream);
+        }
+    };
+    GridBarrier gb{bar, 0u, true};
+    bool alive = true;
+    const bool pending = P.pending_v0 && *P.pending_v0;
+    for (int i = node0; i < S.n_nodes; i += nodes) vbd_predict(S, i, pending, cheb, P.dt, P.inv_dt);
+    int c_begin = __ldg(colour_off), c_end = __ldg(colour_off + 1);
+    gb.arrive();
+    fetch(c_begin + first, c_end);
+    alive = gb.wait(P.error);
+    float omega = 1.f;
+    for (int j = 0; j < iterations && alive; ++j) {
+        for (int c = 0; c < n_colours && alive; ++c) {
+            for (int w = c_begin + first; w < c_end; w += step) {   // sub-block-uniform
+                if (w != c_begin + first) fetch(w, c_end);
+                const bool active = vid >= 0 && S.mask[vid] != 0;
+                if (active && glane == 0) {
+                    asm volatile("prefetch.global.L1 [%0];" ::"l"(S.u_last + vid));
+                    asm volatile("prefetch.global.L1 [%0];" ::"l"(S.y + vid));
+                }
+                float acc[9], cmp[3];
+#pragma unroll
+                for (int k = 0; k < 9; ++k) acc[k] = 0.f;
+#pragma unroll
+                for (int k = 0; k < 3; ++k) cmp[k] = 0.f;
+                while (o < oe) {
+                    float4 cur[EW / 4];
+#pragma unroll
+                    for (int k = 0; k < EW / 4; ++k) cur[k] = nxt[k];
+                    o += t;
+                    if (o < oe) {
+#pragma unroll
+                        for (int k = 0; k < EW / 4; ++k) nxt[k] = ld_hint(S.ent + (size_t)o * (EW / 4) + k, stream);
+                    }
+                    entry_terms<E, MAT, true>(S, reinterpret_cast<const float*>(cur), s_dN, mixed, acc, cmp);
+                }
+                if (mixed) {
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) acc[k] -= cmp[k];
+                }
+                for (int off = t >> 1; off > 0; off >>= 1) {
+#pragma unroll
+                    for (int k = 0; k < 9; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], off);
+                }
+                if (active && glane == 0) vertex_epilogue(S, vid, acc, 0, P, nullptr);
+            }
+            const bool last = c + 1 == n_colours;
+            const int next = last ? 0 : c + 1;
+            c_begin = __ldg(colour_off + next);
+            c_end = __ldg(colour_off + next + 1);
+            gb.arrive();
+            fetch(c_begin + first, c_end);
+            alive = gb.wait(P.error);
+        }
+        const bool fix = j == 0 && S.n_fixed > 0;
+        if (alive && (fix || cheb)) {
+            if (cheb) {
+                if (j == 1) omega = __fdiv_rn(2.f, __fsub_rn(2.f, __fmul_rn(rho, rho)));
+                else if (j > 1) omega = __fdiv_rn(4.f, __fsub_rn(4.f, __fmul_rn(__fmul_rn(rho, rho), omega)));
+                for (int i = node0; i < S.n_nodes; i += nodes) {
+                    if (fix && S.fix_of[i] >= 0) fix_node(S, i, S.fix_of[i]);
+                    chebyshev_node(S, i, j, omega);
+                }
+            } else {
+                for (int k = node0; k < S.n_fixed; k += nodes) fix_node(S, S.fixed[k], S.fixed_group[k]);
+            }
+            gb.arrive();
+            alive = gb.wait(P.error);
+        }
+    }
+    if (alive)
+        for (int i = node0; i < S.n_nodes; i += nodes) vbd_velocity(S, i, P.dt);
+    // every block has left its last barrier once it counts itself here: the last one clears both
+    if (threadIdx.x == 0 && gridDim.x > 1 && atomicAdd(bar + 1, 1u) == gridDim.x - 1) { bar[0] = 0u; bar[1] = 0u; }
+}
+
 // Scripted effects (GPU_Constraint.cu:22-92), run after the fixation in creation order.
 //   crush (kernel_constraint_crush): free nodes flattened to y = 0, last position = position,
 //     velocity 0
@@ -2217,6 +2368,41 @@ void launch_vertex(int element, int material, const SceneDev* scenes, const VWor
         case 7: vertex_mat<7>(material, scenes, work, n_work, form, mode, P, red, st); break;
         case 8: vertex_mat<8>(material, scenes, work, n_work, form, mode, P, red, st); break;
         case 9: vertex_mat<9>(material, scenes, work, n_work, form, mode, P, red, st); break;
+    }
+}
+
+namespace {
+template <int E>
+bool substep_mat(int mat, const SceneDev* scene, const VWork* work, const int* colour_off, int n_colours, int iterations,
+                 float rho, unsigned* bar, int grid, const StepParams& P, cudaStream_t st) {
+    auto go = [&](auto kernel) {
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeCooperative;
+        at[0].val.cooperative = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(grid);
+        cfg.blockDim = dim3(kSubBlocks * kBlock);
+        cfg.stream = st;
+        cfg.attrs = at;
+        cfg.numAttrs = grid > 1 ? 1 : 0;
+        return cudaLaunchKernelEx(&cfg, kernel, scene, work, colour_off, n_colours, iterations, rho, bar, P) == cudaSuccess;
+    };
+    switch (mat) {
+        case 0: return go(k_vbd_substep<E, 0>);
+        case 1: return go(k_vbd_substep<E, 1>);
+        case 2: return go(k_vbd_substep<E, 2>);
+        default: return go(k_vbd_substep<E, 3>);
+    }
+}
+}  // namespace
+
+bool launch_vbd_substep(int element, int material, const SceneDev* scene, const VWork* work, const int* colour_off,
+                        int n_colours, int iterations, float rho, unsigned* bar, int grid, const StepParams& P, cudaStream_t st) {
+    switch (element) {
+        case 3: return substep_mat<3>(material, scene, work, colour_off, n_colours, iterations, rho, bar, grid, P, st);
+        case 6: return substep_mat<6>(material, scene, work, colour_off, n_colours, iterations, rho, bar, grid, P, st);
+        case 7: return substep_mat<7>(material, scene, work, colour_off, n_colours, iterations, rho, bar, grid, P, st);
+        default: return false;
     }
 }
 

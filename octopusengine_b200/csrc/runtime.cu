@@ -28,6 +28,7 @@ using namespace octb;
 
 namespace {
 constexpr int kBlockThreads = 128;
+constexpr int kSubBlocks = 4;   // k_vbd_substep: groups of kBlockThreads per block
 
 // NVTX ranges around frames, sub-steps and colour sweeps (host side; a profiler shows them on
 // the timeline, and without one they cost a pointer test).
@@ -48,6 +49,7 @@ struct oct_ctx {
     float last_ms = 0.f;
     uint64_t launches = 0;
     bool tables[10] = {false};
+    int sms = 0;         // streaming multiprocessors (sm_count)
     std::mutex mu;       // guards the budget accounting and the shape-table upload
     std::mutex err_mu;   // guards err (scenes may be created from several host threads)
     // device blocks released by destroyed scenes and batches, kept for reuse (size -> pointer):
@@ -171,6 +173,9 @@ struct oct_scene {
     VWork* d_vwork = nullptr;
     std::vector<int> vwork_off;     // per colour: [vwork_off[c], vwork_off[c+1])
     std::vector<int> form;          // per colour: launch_form
+    int* d_vwork_off = nullptr;
+    int max_items = 0;              // most work items of a colour
+    unsigned* d_bar = nullptr;      // grid barrier of the one-launch sub-step
     NWork* d_nwork = nullptr;
     int n_nwork = 0;
     NWork* d_fwork = nullptr;
@@ -387,14 +392,17 @@ oct_status build_vertex_work(oct_scene* s) {
     std::vector<VWork> vw;
     s->vwork_off.assign(1, 0);
     s->form.clear();
+    s->max_items = 0;
     for (int k = 0; k + 1 < (int)s->color_off.size(); ++k) {
         const int begin = s->color_off[k], end = s->color_off[k + 1];
         const ColourLanes l = colour_lanes(s->element, s->tpv, begin, end, s->own_off);
         s->form.push_back(launch_form(s->element, s->tpv, (int64_t)s->own_off[end] - s->own_off[begin]));
         append_vwork(vw, 0, s->element, begin, end, s->form[k], l, lane_div((int64_t)l.width * (end - begin)), s->own_off);
         s->vwork_off.push_back((int)vw.size());
+        s->max_items = std::max(s->max_items, s->vwork_off[k + 1] - s->vwork_off[k]);
     }
-    return upload(s->ctx, s->mem, s->d_vwork, vw);
+    oct_status st = upload(s->ctx, s->mem, s->d_vwork, vw);
+    return st ? st : upload(s->ctx, s->mem, s->d_vwork_off, s->vwork_off);
 }
 
 oct_status build_scene(oct_ctx* c, const oct_scene_desc* d, oct_scene* s);
@@ -869,6 +877,7 @@ oct_status build_scene(oct_ctx* c, const oct_scene_desc* d, oct_scene* s) {
     s->pending_host = s->has_v0 && d->solver == OCT_SOLVER_VBD ? 1 : 0;
     if ((st = upload(c, s->mem, s->d_pending, std::vector<int>{s->pending_host}))) return st;
     if ((st = s->mem.alloc(s->d_red, 4))) return st;
+    if ((st = upload(c, s->mem, s->d_bar, std::vector<unsigned>(2, 0u)))) return st;
     if (d->solver == OCT_SOLVER_EXPLICIT && (st = s->mem.alloc(s->d_contrib, (size_t)E * NE))) return st;
 
     // work tables
@@ -909,6 +918,23 @@ void enqueue_effects(oct_scene* s, float dt, cudaStream_t st) {
     }
 }
 
+int sm_count(oct_ctx* c) {
+    if (!c->sms) cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->device);
+    return c->sms;
+}
+
+// Whether the scene's VBD sub-step runs as one cooperative launch (k_vbd_substep): lane-group
+// items with owner entries, in place and in ascending colour order, nothing between the sweeps but
+// the fixation and Chebyshev, and colours of at most two items per SM, above which the work in a
+// colour outweighs its launch (per colour, one launch / a launch each: P1 45 nodes 1.9 / 3.7 us,
+// 2,025 nodes 3.1 / 3.9, 35,721 nodes 5.4 / 6.2; Q1 45 nodes 2.2 / 3.9, 18,785 nodes 3.9 / 5.1; P2
+// 2,025 nodes 3.3 / 4.5, 40,625 nodes 4.4 / 5.5; P2 140,481 nodes, 308 items, a frame of five
+// sub-steps 4.56 / 4.38 ms).
+bool one_launch(const oct_scene* s) {
+    return s->max_items <= 2 * sm_count(s->ctx) && s->tpv > 0 && (s->element == kTetra || s->element == kHexa || s->element == kTetra10) && s->h.ent &&
+           s->in_place && s->order_mode == OCT_ORDER_ASCENDING && !s->mg_sub && !s->n_effects && !s->box;
+}
+
 // One GPU_VBD::step (octopus/src/GPU/VBD/GPU_VBD.cu:38-61) of one scene with the reference's
 // launch structure: predictor, iterations x (one launch per colour [+ commit] + constraints
 // [+ Chebyshev]), velocity update.  The fixation runs in the sub-step's first iteration only:
@@ -932,6 +958,15 @@ void vbd_substep(oct_scene* s, float dt) {
         cudaMemsetAsync(s->d_pending, 0, sizeof(int), st);
         s->pending_host = 0;
     };
+    if (one_launch(s)) {
+        const int sms = sm_count(c);
+        const int grid = s->max_items <= 2 * kSubBlocks ? 1 : std::min(s->max_items, sms);
+        launch_vbd_substep(s->element, s->material, s->d_scene, s->d_vwork, s->d_vwork_off, s->n_colors, s->iterations,
+                           cheb ? s->rho : 0.f, s->d_bar, grid, P, st);
+        c->launches++;
+        consumed();
+        return;
+    }
     launch_predict(s->d_scene, s->d_nwork, s->n_nwork, 0, 0, cheb ? 1 : 0, P, st);
     c->launches++;
     consumed();
