@@ -17,8 +17,8 @@
 //
 // Colour-sorted vertex slots: vids[slot] is the node solved in that slot; slots of colour
 // c are [color_off[c], color_off[c+1]) in ascending node id (GPU_VBD_FEM::create_buffers,
-// octopus/src/GPU/VBD/GPU_VBD_FEM.cu:594-675); own_off/owners is the owner CSR in slot
-// order with owners packed as (element id << 5) | local node index.
+// octopus/src/GPU/VBD/GPU_VBD_FEM.cu:594-675); owners is the owner CSR in slot order
+// (slots holds each slot's part of it) with owners packed as (element id << 5) | local node index.
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -62,11 +62,12 @@ struct SceneDev {
     const float4* eq;   // n_elements * NQ * 3
     const int* vids;    // n_nodes, colour-sorted
     const int4* slots;  // the same slots with their owners: node, first owner, owner count, 0
-    const int* own_off; // n_nodes + 1, slot order
     const int* owners;  // packed (eid << 5) | r
     const int* fixed;   // n_fixed node ids
     const int* fixed_group;            // n_fixed rigid-group indices
-    const int* fix_of;                 // explicit: per node its rigid group if fixed, else -1 (or null)
+    const int* fix_of;                 // VBD, explicit: per node its rigid group if fixed, else -1 (or null)
+    const int* topo_t;                 // explicit: the topology node by node, [local node][element]
+    const int* owner_at;               // explicit: place of (element, local node) in owners, [local node][element]
     const float* fix;                  // kFixGroups x 16: com (3), offset (3), rotation (9, column-major), pad
     int n_nodes, n_elements, n_fixed, element;
     int eq_stride;                     // records per element: NQ, or 1 for affine elements

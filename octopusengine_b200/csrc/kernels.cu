@@ -279,6 +279,15 @@ __device__ __forceinline__ void hex_q1_coefficients(const float* ux, const float
     h.z = (me1 + me0) * s;   h.xz = (me1 - me0) * s;  h.yz = (mo1 + mo0) * s;   h.xyz = (mo1 - mo0) * s;
 }
 
+// Jx at Gauss point q, at (s_q0, s_q1, s_q2) / sqrt(3), s_q the signs of node q.
+__device__ __forceinline__ void hex_q1_jacobian(const HexCoef& hc, int q, V3& J0, V3& J1, V3& J2) {
+    constexpr float c = 0.57735026918962576f;
+    const float xi = c * kHexSign[q][0], et = c * kHexSign[q][1], ze = c * kHexSign[q][2];
+    J0 = hc.x + hc.xy * et + hc.xz * ze + hc.xyz * (et * ze);
+    J1 = hc.y + hc.xy * xi + hc.yz * ze + hc.xyz * (xi * ze);
+    J2 = hc.z + hc.xz * xi + hc.yz * et + hc.xyz * (xi * et);
+}
+
 // P2 (Tetra_10) Jx from its barycentric structure.  With L = (1 - xi - eta - zeta, xi, eta,
 // zeta), du/dxi_k = D_k - D_0 where D_i = du/dL_i = (4 L_i - 1) u_i + 4 sum_j L_j u_ij (u_ij the
 // edge node between corners i and j) is linear in L.  The 4-point rule puts L = b at one corner
@@ -366,12 +375,7 @@ __device__ __forceinline__ void element_terms(const float* ux, const float* uy, 
         // Jx columns: Jk = sum_i u_i dN_qi[k]
         V3 J0 = mk(0, 0, 0), J1 = mk(0, 0, 0), J2 = mk(0, 0, 0);
         if constexpr (E == 6) {
-            // Gauss point q sits at (s_q0, s_q1, s_q2) / sqrt(3), s_q the signs of node q
-            constexpr float c = 0.57735026918962576f;
-            const float xi = c * kHexSign[q][0], et = c * kHexSign[q][1], ze = c * kHexSign[q][2];
-            J0 = hc.x + hc.xy * et + hc.xz * ze + hc.xyz * (et * ze);
-            J1 = hc.y + hc.xy * xi + hc.yz * ze + hc.xyz * (xi * ze);
-            J2 = hc.z + hc.xz * xi + hc.yz * et + hc.xyz * (xi * et);
+            hex_q1_jacobian(hc, q, J0, J1, J2);
         } else if constexpr (E == 7) {
             p2_jacobian(ux, uy, uz, p2, q, J0, J1, J2);
         } else {
@@ -1638,6 +1642,8 @@ __device__ __forceinline__ void xpbd_pair(int m, V3 F0, V3 F1, V3 F2, float lam,
     }
 }
 
+// Lanes per element of the explicit group kernel: at least one per quadrature point.
+template <int E> struct ElemLanes { static constexpr int G = E == 3 ? 4 : (E == 6 || E == 7 ? 8 : (E == 8 ? 16 : 32)); };
 // lanes per element: at least one per quadrature point
 template <int E> struct XpbdLanes { static constexpr int G = E == 3 ? 4 : (E == 6 || E == 7 ? 8 : (E == 8 ? 16 : 32)); };
 
@@ -1878,7 +1884,9 @@ __device__ __forceinline__ void pk1_tilde(V3 F0, V3 F1, V3 F2, float lam, float 
 template <int E, int MAT>
 __global__ void __launch_bounds__(kBlock) k_explicit_elem(const SceneDev* __restrict__ scenes, int n_elements,
                                                           float4* __restrict__ contrib, StepParams P) {
-    constexpr int NE = ElemT<E>::NE, NQ = ElemT<E>::NQ, G = XpbdLanes<E>::G, GPB = kBlock / G;
+    // contributions go to the owner's place in slot order (SceneDev::owner_at), read in order by
+    // k_explicit_gather
+    constexpr int NE = ElemT<E>::NE, NQ = ElemT<E>::NQ, G = ElemLanes<E>::G, GPB = kBlock / G;
     constexpr int NI = (NE + G - 1) / G;   // nodes per lane
     static_assert(NQ <= G, "one quadrature point per lane");
     __shared__ __align__(16) float s_dN[((NQ * NE * 3 + 3) / 4) * 4];
@@ -1944,7 +1952,7 @@ __global__ void __launch_bounds__(kBlock) k_explicit_elem(const SceneDev* __rest
                 fy -= t0.y * dr[0] + t1.y * dr[1] + t2.y * dr[2];
                 fz -= t0.z * dr[0] + t1.z * dr[1] + t2.z * dr[2];
             }
-            contrib[(size_t)eid * NE + i] = make_float4(fx, fy, fz, 0.f);
+            contrib[S.owner_at[(size_t)i * n_elements + eid]] = make_float4(fx, fy, fz, 0.f);
         }
         return;
     }
@@ -1974,39 +1982,167 @@ __global__ void __launch_bounds__(kBlock) k_explicit_elem(const SceneDev* __rest
         f.y = acc[1] - kd * (acc[4] * vv.x + acc[6] * vv.y + acc[7] * vv.z);
         f.z = acc[2] - kd * (acc[5] * vv.x + acc[7] * vv.y + acc[8] * vv.z);
         f.w = 0.f;
-        contrib[(size_t)eid * NE + i] = f;
+        contrib[S.owner_at[(size_t)i * n_elements + eid]] = f;
     }
 }
 
-// Per node: the sum of its owners' element contributions in owner order (compensated in
-// mixed precision), kept in u_new (the force buffer of the explicit solver), then the
-// semi-implicit Euler update of that node (kenerl_semi_exicit_integration,
-// octopus/src/GPU/GPU_Integrator.cu:27-34; the arithmetic of k_predict kind 1) and, for a
-// fixed node, its fixation (fix_node, as k_constraints).  work indexes
-// the scene's slots (one colour: every node).
-__global__ void k_explicit_gather(const SceneDev* __restrict__ scenes, const NWork* __restrict__ work,
-                                  const float4* __restrict__ contrib, int ne, StepParams P) {
-    pdl_trigger();
+// Blocks of 64: at 96 (P2) to 128 (Q1) registers a block is a tenth of an SM, which keeps the last
+// wave small (98,304 P2 elements: sub-step 16.5 us with 64, 17.0 with 128; 1,920 P2 elements 7.2
+// against 9.4 us).
+constexpr int kElemBlock = 64;
+// One thread per element (P1, Q1, P2 without damping): the group kernel above spent its time on
+// blocks of 16 elements that each staged the table and passed everything through shared memory
+// (6,144 blocks for 98,304 P2 elements).  Here a thread holds its element: node ids, owner places
+// and record load before the wait, F at every point comes from the element's structure (P2
+// barycentric, Q1 monomials), and the nodal forces are the adjoint of that structure: per point
+// a few sums into its coefficients, distributed to the nodes once.
+template <int E, int MAT>
+__global__ void __launch_bounds__(kElemBlock) k_explicit_thread(const SceneDev* __restrict__ scene, int n_elements,
+                                                                           float4* __restrict__ contrib) {
+    constexpr int NE = ElemT<E>::NE, NQ = ElemT<E>::NQ;
+    const SceneDev& S = *scene;
+    const int e = blockIdx.x * kElemBlock + threadIdx.x;
+    const bool on = e < n_elements;
+    const unsigned long long keep = policy_keep();
+    int id[NE], at[NE];
+#pragma unroll
+    for (int i = 0; i < NE; ++i) {
+        id[i] = on ? __ldg(S.topo_t + (size_t)i * n_elements + e) : 0;
+        at[i] = on ? __ldg(S.owner_at + (size_t)i * n_elements + e) : 0;
+    }
+    const bool affine = S.eq_stride == 1;
+    const float4* rec = S.eq + (size_t)(on ? e : 0) * S.eq_stride * 3;
+    float4 A = __ldg(rec), B = __ldg(rec + 1), C = __ldg(rec + 2);
     pdl_wait();
-    const NWork wk = work[blockIdx.x];
-    if ((int)threadIdx.x >= wk.count) return;
-    const SceneDev& S = scenes[wk.scene];
-    const int slot = wk.begin + threadIdx.x;
-    const int vid = S.vids[slot];
-    const int ob = S.own_off[slot], oe = S.own_off[slot + 1];
+    if (!on) return;
+    float ux[NE], uy[NE], uz[NE];
+#pragma unroll
+    for (int i = 0; i < NE; ++i) {
+        const float4 t = ld_hint(&S.u[id[i]], keep);
+        ux[i] = t.x; uy[i] = t.y; uz[i] = t.z;
+    }
+    V3 f[NE];
+#pragma unroll
+    for (int i = 0; i < NE; ++i) f[i] = mk(0, 0, 0);
+    [[maybe_unused]] HexCoef hc, hg;
+    if constexpr (E == 6) {
+        hex_q1_coefficients(ux, uy, uz, hc);
+        hg.x = hg.y = hg.z = hg.xy = hg.xz = hg.yz = hg.xyz = mk(0, 0, 0);
+    }
+    [[maybe_unused]] P2Base p2;
+    [[maybe_unused]] V3 g1 = mk(0, 0, 0), g2 = g1, g3 = g1;   // P2: sums of P~'s columns
+    if constexpr (E == 7) p2_base(ux, uy, uz, p2);
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        if (!affine && q > 0) { A = __ldg(rec + 3 * q); B = __ldg(rec + 3 * q + 1); C = __ldg(rec + 3 * q + 2); }
+        V3 J0, J1, J2;
+        if constexpr (E == 3) {
+            const V3 u0 = mk(ux[0], uy[0], uz[0]);
+            J0 = mk(ux[1], uy[1], uz[1]) - u0; J1 = mk(ux[2], uy[2], uz[2]) - u0; J2 = mk(ux[3], uy[3], uz[3]) - u0;
+        } else if constexpr (E == 6) {
+            hex_q1_jacobian(hc, q, J0, J1, J2);
+        } else {
+            p2_jacobian(ux, uy, uz, p2, q, J0, J1, J2);
+        }
+        const V3 m0 = mk(A.x, A.y, A.z), m1 = mk(A.w, B.x, B.y), m2 = mk(B.z, B.w, C.x);
+        V3 F0 = J0 * m0.x + J1 * m0.y + J2 * m0.z;
+        V3 F1 = J0 * m1.x + J1 * m1.y + J2 * m1.z;
+        V3 F2 = J0 * m2.x + J1 * m2.y + J2 * m2.z;
+        F0.x += 1.f; F1.y += 1.f; F2.z += 1.f;
+        V3 T0, T1, T2;
+        pk1_tilde<MAT>(F0, F1, F2, C.z, C.w, C.y * wq<E>(q), m0, m1, m2, T0, T1, T2);
+        if constexpr (E == 3) {
+            f[1] = T0; f[2] = T1; f[3] = T2;
+            f[0] = (T0 + T1 + T2) * -1.f;
+        } else if constexpr (E == 6) {
+            constexpr float c = 0.57735026918962576f;
+            const float xi = c * kHexSign[q][0], et = c * kHexSign[q][1], ze = c * kHexSign[q][2];
+            hg.x = hg.x + T0; hg.y = hg.y + T1; hg.z = hg.z + T2;
+            hg.xy = hg.xy + T0 * et + T1 * xi; hg.xz = hg.xz + T0 * ze + T2 * xi; hg.yz = hg.yz + T1 * ze + T2 * et;
+            hg.xyz = hg.xyz + T0 * (et * ze) + T1 * (xi * ze) + T2 * (xi * et);
+        } else {
+            // J_k = R_k + c (w_k - w_0): w_i is node i at its own corner p, else edge node (i, p)
+            constexpr float c = (float)(4 * (kP2b - kP2a));
+            const int p = (q + 1) & 3;
+            const V3 t[4] = {(T0 + T1 + T2) * -1.f, T0, T1, T2};
+            g1 = g1 + T0; g2 = g2 + T1; g3 = g3 + T2;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int n = i == p ? i : p2_edge_node(i, p);
+                f[n] = f[n] + t[i] * c;
+            }
+        }
+    }
+    if constexpr (E == 6) {
+        constexpr float s = 0.125f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float sx = s * kHexSign[i][0], sy = s * kHexSign[i][1], sz = s * kHexSign[i][2];
+            const float sxy = s * (kHexSign[i][0] * kHexSign[i][1]), sxz = s * (kHexSign[i][0] * kHexSign[i][2]),
+                        syz = s * (kHexSign[i][1] * kHexSign[i][2]),
+                        sxyz = s * (kHexSign[i][0] * kHexSign[i][1] * kHexSign[i][2]);
+            f[i] = hg.x * sx + hg.y * sy + hg.z * sz + hg.xy * sxy + hg.xz * sxz + hg.yz * syz + hg.xyz * sxyz;
+        }
+    } else if constexpr (E == 7) {
+        // R_k = Pa_k - Pa_0, Pa_i = ca u_i + cs (sum of the edge nodes at corner i)
+        constexpr float ca = (float)(4 * kP2a - 1), cs = (float)(4 * kP2a);
+        const V3 pa[4] = {(g1 + g2 + g3) * -1.f, g1, g2, g3};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            f[i] = f[i] + pa[i] * ca;
+#pragma unroll
+            for (int k = i + 1; k < 4; ++k) f[p2_edge_node(i, k)] = f[p2_edge_node(i, k)] + (pa[i] + pa[k]) * cs;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < NE; ++i) contrib[at[i]] = make_float4(-f[i].x, -f[i].y, -f[i].z, 0.f);
+    pdl_trigger();   // at the end (blocks waiting in this one's place cost P1 9.1 -> 6.8 us per sub-step)
+}
+
+// Per node: the sum of its owners' contributions (compensated in mixed precision), kept in u_new
+// (the force buffer of the explicit solver), then the semi-implicit Euler update of that node
+// (kenerl_semi_exicit_integration, octopus/src/GPU/GPU_Integrator.cu:27-34; the arithmetic of
+// k_predict kind 1) and, for a fixed node, its fixation (fix_node, as k_constraints).  A node's
+// contributions are contiguous, and four lanes read them together (64 bytes at a time); the slot
+// loads before the wait.
+constexpr int kGatherLanes = 4;
+
+__global__ void k_explicit_gather(const SceneDev* __restrict__ scene, const float4* __restrict__ contrib, StepParams P) {
+    const SceneDev& S = *scene;
+    const int g = blockIdx.x * blockDim.x + threadIdx.x, slot = g / kGatherLanes, lane = g % kGatherLanes;
+    const bool on = slot < S.n_nodes;   // no early exit: the group shuffles
+    const int4 sl = on ? __ldg(S.slots + slot) : make_int4(0, 0, 0, 0);
+    const int vid = sl.x;
     const bool mixed = S.precision != 0;
+    const int group = on && S.fix_of ? __ldg(S.fix_of + vid) : -1;
+    pdl_wait();
     float fx = 0.f, fy = 0.f, fz = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
-    for (int o = ob; o < oe; ++o) {
-        const int packed = __ldg(S.owners + o);
-        const float4 c = contrib[(size_t)(packed >> kOwnerShift) * ne + (packed & ((1 << kOwnerShift) - 1))];
+    float4 u, v, y;
+    if (on && lane == 0) { u = S.u[vid]; v = S.v[vid]; y = S.y[vid]; }
+#pragma unroll 4
+    for (int o = lane; o < sl.z; o += kGatherLanes) {
+        const float4 c = contrib[sl.y + o];
         if (mixed) { kadd(fx, cx, c.x); kadd(fy, cy, c.y); kadd(fz, cz, c.z); }
         else { fx += c.x; fy += c.y; fz += c.z; }
     }
+#pragma unroll
+    for (int off = 1; off < kGatherLanes; off <<= 1) {
+        const float ox = __shfl_xor_sync(0xffffffffu, fx, off), oy = __shfl_xor_sync(0xffffffffu, fy, off),
+                    oz = __shfl_xor_sync(0xffffffffu, fz, off);
+        if (mixed) {   // both sums and both compensations
+            const float ex = __shfl_xor_sync(0xffffffffu, cx, off), ey = __shfl_xor_sync(0xffffffffu, cy, off),
+                        ez = __shfl_xor_sync(0xffffffffu, cz, off);
+            kadd(fx, cx, ox); kadd(fy, cy, oy); kadd(fz, cz, oz);
+            cx += ex; cy += ey; cz += ez;
+        } else {
+            fx += ox; fy += oy; fz += oz;
+        }
+    }
+    if (!on || lane != 0) return;
     if (mixed) { fx -= cx; fy -= cy; fz -= cz; }
     S.u_new[vid] = make_float4(fx, fy, fz, 0.f);
     const float dt = P.dt;
-    float4 u = S.u[vid], v = S.v[vid];
-    const float w = 1.f / S.y[vid].w;
+    const float w = 1.f / y.w;
     S.u_last[vid] = u;
     v.x += (S.gx + fx * w) * dt; v.y += (S.gy + fy * w) * dt; v.z += (S.gz + fz * w) * dt;
     u.x += v.x * dt; u.y += v.y * dt; u.z += v.z * dt;
@@ -2015,10 +2151,8 @@ __global__ void k_explicit_gather(const SceneDev* __restrict__ scenes, const NWo
     if (!isfinite(u.x + u.y + u.z + v.x + v.y + v.z)) atomicOr(S.status, kStatusNonFinite);
     // then the fixation of the sub-step (GPU_SemiExplicit::step applies the constraints after
     // the integration): fixed nodes are set to their group's target
-    if (S.fix_of) {
-        const int g = S.fix_of[vid];
-        if (g >= 0) fix_node(S, vid, g);
-    }
+    if (group >= 0) fix_node(S, vid, group);
+    pdl_trigger();
 }
 
 template <int E>
@@ -2467,31 +2601,41 @@ void launch_xpbd(int element, int material, bool raw, const SceneDev* scenes, co
 
 namespace {
 template <int E>
-void explicit_mat(int mat, const SceneDev* scenes, int n_elements, float4* contrib, const StepParams& P, cudaStream_t st) {
-    const int grid = (n_elements + kBlock / XpbdLanes<E>::G - 1) / (kBlock / XpbdLanes<E>::G);
+void explicit_mat(int mat, bool damped, const SceneDev* scene, int n_elements, float4* contrib, const StepParams& P, cudaStream_t st) {
+    if constexpr (E == 3 || E == 6 || E == 7) {
+        if (!damped) {
+            const int grid = (n_elements + kElemBlock - 1) / kElemBlock;
+            switch (mat) {
+                case 0: launch_pdl(k_explicit_thread<E, 0>, grid, kElemBlock, 0, st, scene, n_elements, contrib); return;
+                case 1: launch_pdl(k_explicit_thread<E, 1>, grid, kElemBlock, 0, st, scene, n_elements, contrib); return;
+                case 2: launch_pdl(k_explicit_thread<E, 2>, grid, kElemBlock, 0, st, scene, n_elements, contrib); return;
+                default: launch_pdl(k_explicit_thread<E, 3>, grid, kElemBlock, 0, st, scene, n_elements, contrib); return;
+            }
+        }
+    }
+    const int grid = (n_elements + kBlock / ElemLanes<E>::G - 1) / (kBlock / ElemLanes<E>::G);
     switch (mat) {
-        case 0: launch_pdl(k_explicit_elem<E, 0>, grid, kBlock, 0, st, scenes, n_elements, contrib, P); break;
-        case 1: launch_pdl(k_explicit_elem<E, 1>, grid, kBlock, 0, st, scenes, n_elements, contrib, P); break;
-        case 2: launch_pdl(k_explicit_elem<E, 2>, grid, kBlock, 0, st, scenes, n_elements, contrib, P); break;
-        default: launch_pdl(k_explicit_elem<E, 3>, grid, kBlock, 0, st, scenes, n_elements, contrib, P); break;
+        case 0: launch_pdl(k_explicit_elem<E, 0>, grid, kBlock, 0, st, scene, n_elements, contrib, P); break;
+        case 1: launch_pdl(k_explicit_elem<E, 1>, grid, kBlock, 0, st, scene, n_elements, contrib, P); break;
+        case 2: launch_pdl(k_explicit_elem<E, 2>, grid, kBlock, 0, st, scene, n_elements, contrib, P); break;
+        default: launch_pdl(k_explicit_elem<E, 3>, grid, kBlock, 0, st, scene, n_elements, contrib, P); break;
     }
 }
 }  // namespace
 
-void launch_explicit_force(int element, int material, const SceneDev* scene, int n_elements, float4* contrib,
-                           const NWork* slots, int n_slots, const StepParams& P, cudaStream_t st) {
+void launch_explicit_force(int element, int material, bool damped, const SceneDev* scene, int n_nodes, int n_elements,
+                           float4* contrib, const StepParams& P, cudaStream_t st) {
     if (n_elements <= 0) return;
     switch (element) {
-        case 3: explicit_mat<3>(material, scene, n_elements, contrib, P, st); break;
-        case 6: explicit_mat<6>(material, scene, n_elements, contrib, P, st); break;
-        case 7: explicit_mat<7>(material, scene, n_elements, contrib, P, st); break;
-        case 8: explicit_mat<8>(material, scene, n_elements, contrib, P, st); break;
-        case 9: explicit_mat<9>(material, scene, n_elements, contrib, P, st); break;
+        case 3: explicit_mat<3>(material, damped, scene, n_elements, contrib, P, st); break;
+        case 6: explicit_mat<6>(material, damped, scene, n_elements, contrib, P, st); break;
+        case 7: explicit_mat<7>(material, damped, scene, n_elements, contrib, P, st); break;
+        case 8: explicit_mat<8>(material, damped, scene, n_elements, contrib, P, st); break;
+        case 9: explicit_mat<9>(material, damped, scene, n_elements, contrib, P, st); break;
         default: return;
     }
-    if (n_slots > 0)
-        launch_pdl(k_explicit_gather, n_slots, kNodeChunk, 0, st, scene, slots, (const float4*)contrib,
-                   element == 3 ? 4 : element == 6 ? 8 : element == 7 ? 10 : element == 8 ? 20 : 27, P);
+    constexpr int kNodes = 256 / kGatherLanes;
+    launch_pdl(k_explicit_gather, (n_nodes + kNodes - 1) / kNodes, 256, 0, st, scene, (const float4*)contrib, P);
 }
 
 int point_item_pairs(int element) { return element == 8 ? point_slots<8>() : point_slots<9>(); }

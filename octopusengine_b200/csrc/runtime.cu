@@ -743,10 +743,10 @@ oct_status build_scene(oct_ctx* c, const oct_scene_desc* d, oct_scene* s) {
     if (s->rho > 0.f) {
         if ((st = upload(c, s->mem, p1, zero4)) || (st = upload(c, s->mem, p2, zero4))) return st;
     }
-    int *maskd, *topod, *vidsd, *offd, *ownd, *fixd = nullptr;
+    int *maskd, *topod, *vidsd, *ownd, *fixd = nullptr;
     float4* eqd;
     if ((st = upload(c, s->mem, maskd, mask)) || (st = upload(c, s->mem, topod, topo)) || (st = upload(c, s->mem, eqd, eq)) ||
-        (st = upload(c, s->mem, vidsd, slot_vids)) || (st = upload(c, s->mem, offd, own_off)) || (st = upload(c, s->mem, ownd, owners)))
+        (st = upload(c, s->mem, vidsd, slot_vids)) || (st = upload(c, s->mem, ownd, owners)))
         return st;
     std::vector<int4> slots(N);
     for (int sl = 0; sl < N; ++sl) slots[sl] = make_int4(slot_vids[sl], own_off[sl], own_off[sl + 1] - own_off[sl], 0);
@@ -757,7 +757,7 @@ oct_status build_scene(oct_ctx* c, const oct_scene_desc* d, oct_scene* s) {
     if (s->n_fixed && ((st = upload(c, s->mem, fixd, s->fixed)) || (st = upload(c, s->mem, fgd, s->fixed_group)))) return st;
     if ((st = upload(c, s->mem, s->d_fix, std::vector<float>(s->fix_host, s->fix_host + kFixGroups * 16)))) return st;
     h.u = u; h.u_last = ul; h.y = y; h.v = v; h.u_new = un; h.prev1 = p1; h.prev2 = p2; h.mask = maskd; h.X = Xd;
-    h.topo = topod; h.eq = eqd; h.vids = vidsd; h.own_off = offd; h.owners = ownd; h.fixed = fixd;
+    h.topo = topod; h.eq = eqd; h.vids = vidsd; h.owners = ownd; h.fixed = fixd;
     h.fixed_group = fgd; h.fix = s->d_fix;
     if (d->solver != OCT_SOLVER_XPBD && s->n_fixed) {   // for the updates that apply the fixation node by node
         std::vector<int32_t> fix_of(N, -1);
@@ -765,6 +765,17 @@ oct_status build_scene(oct_ctx* c, const oct_scene_desc* d, oct_scene* s) {
         int* fod;
         if ((st = upload(c, s->mem, fod, fix_of))) return st;
         h.fix_of = fod;
+    }
+    if (d->solver == OCT_SOLVER_EXPLICIT) {
+        std::vector<int32_t> topo_t((size_t)E * NE), owner_at((size_t)E * NE);
+        for (int e = 0; e < E; ++e)
+            for (int j = 0; j < NE; ++j) topo_t[(size_t)j * E + e] = d->topology[(size_t)e * NE + j];
+        for (size_t o = 0; o < owners.size(); ++o)
+            owner_at[(size_t)(owners[o] & ((1 << kOwnerShift) - 1)) * E + (owners[o] >> kOwnerShift)] = (int32_t)o;
+        int *ttd, *oad;
+        if ((st = upload(c, s->mem, ttd, topo_t)) || (st = upload(c, s->mem, oad, owner_at))) return st;
+        h.topo_t = ttd;
+        h.owner_at = oad;
     }
     h.n_nodes = N; h.n_elements = E; h.n_fixed = s->n_fixed; h.element = d->element;
     h.damping = d->damping;
@@ -1055,7 +1066,7 @@ void explicit_substep(oct_scene* s, float dt) {
     StepParams P = base_params(c, dt);
     // element-centric force pass, then per node the sum over its owners and the semi-implicit
     // Euler update (GPU_FEM_Explicit::step then GPU_SemiExplicit's integration)
-    launch_explicit_force(s->element, s->material, s->d_scene, s->n_elements, s->d_contrib, s->d_nwork, s->n_nwork, P, st);
+    launch_explicit_force(s->element, s->material, s->h.damping != 0.f, s->d_scene, s->n_nodes, s->n_elements, s->d_contrib, P, st);
     c->launches += 2;   // the fixation runs inside the update kernel (SceneDev::fix_of)
     enqueue_effects(s, dt, st);
     if (s->box) { launch_constraints(s->d_scene, s->d_nwork, s->n_nwork, 1, st); c->launches++; }
@@ -1178,7 +1189,8 @@ oct_status oct_scene_footprint(const oct_scene_desc* d, size_t* bytes) {
     b += E * ne * sizeof(int) * 2 + E * nq * 3 * sizeof(float4);   // topology, owners, quadrature records
     b += E * ne * (size_t)entry_words(ne) * sizeof(float);                  // owner entries
     b += (ne == 4 ? 4 : 1) * E * 3 * sizeof(float4);                        // distinct records, at most
-    if (d->solver == OCT_SOLVER_EXPLICIT) b += E * ne * sizeof(float4) + N * sizeof(int);   // contributions, fixation map
+    if (d->solver == OCT_SOLVER_EXPLICIT) b += E * ne * (sizeof(float4) + 2 * sizeof(int));   // contributions, their places, topology
+    if (d->solver != OCT_SOLVER_XPBD) b += N * sizeof(int);                                   // fixation map
     b += (N / 16 + 64) * sizeof(VWork) + (N / 256 + 8) * 2 * sizeof(NWork) + (size_t)std::max(d->n_fixed, 0) * sizeof(int);
     if (d->solver == OCT_SOLVER_XPBD) b += E * (ne + 1) * sizeof(int);   // colour-sorted element ids and topology
     b += 4096;   // descriptors and reduction scratch
