@@ -1644,8 +1644,15 @@ __device__ __forceinline__ void xpbd_pair(int m, V3 F0, V3 F1, V3 F2, float lam,
 
 // Lanes per element of the explicit group kernel: at least one per quadrature point.
 template <int E> struct ElemLanes { static constexpr int G = E == 3 ? 4 : (E == 6 || E == 7 ? 8 : (E == 8 ? 16 : 32)); };
-// lanes per element: at least one per quadrature point
-template <int E> struct XpbdLanes { static constexpr int G = E == 3 ? 4 : (E == 6 || E == 7 ? 8 : (E == 8 ? 16 : 32)); };
+// Lanes per element and block size of the XPBD kernel.  P2 has four points and ten nodes: with
+// eight lanes half of them idled at the points and a second round moved two nodes.  P1 blocks are
+// of 64 threads, so that a colour of one scene spreads over more SMs.  With the loads before the
+// wait, per colour: P2 4,000 elements 5.35 -> 4.14 us, P1 4,100 elements 4.48 -> 3.25 us; a batch of
+// 64 mixed scenes 822 -> 669 us per sub-step.
+template <int E> struct XpbdLanes {
+    static constexpr int G = E == 7 ? 4 : ElemLanes<E>::G;
+    static constexpr int kThreads = E == 3 ? 64 : kBlock;
+};
 
 template <int G> __device__ __forceinline__ float group_sum(float v) {
 #pragma unroll
@@ -1658,41 +1665,37 @@ template <int G> __device__ __forceinline__ float group_sum(float v) {
 // registers) serves batched launches of several waves, whose time is set by how many elements
 // are in flight: the 256-scene XPBD frame 17.05 -> 15.65 ms, against a single P2 scene's frame
 // 0.889 -> 0.989 ms with 6 blocks.
+//
+// Nothing a step writes is read before pdl_wait() but everything else is: the work item, node ids,
+// inverse masses and the quadrature record load under the previous colour's tail (a colour of
+// 4,000 elements is a chain of dependent loads more than it is work).
 template <int E, int MAT, bool RAW, int MINB>
-__global__ void __launch_bounds__(kBlock, MINB) k_xpbd(const SceneDev* __restrict__ scenes, const XWork* __restrict__ work,
-                                                 StepParams P) {
-    constexpr int NE = ElemT<E>::NE, NQ = ElemT<E>::NQ, G = XpbdLanes<E>::G, GPB = kBlock / G;
+__global__ void __launch_bounds__(XpbdLanes<E>::kThreads, MINB * kBlock / XpbdLanes<E>::kThreads)
+k_xpbd(const SceneDev* __restrict__ scenes, const XWork* __restrict__ work, StepParams P) {
+    constexpr int NE = ElemT<E>::NE, NQ = ElemT<E>::NQ, G = XpbdLanes<E>::G, GPB = XpbdLanes<E>::kThreads / G;
     constexpr int NI = (NE + G - 1) / G;   // nodes per lane
     static_assert(NQ <= G, "one quadrature point per lane");
     __shared__ __align__(16) float s_dN[((NQ * NE * 3 + 3) / 4) * 4];
-    __shared__ __align__(16) float4 s_pos[GPB][NE];
-    __shared__ __align__(16) float4 s_P[GPB][NQ][3];
+    // rows of an odd number of float4, so that the groups of a warp fall on different banks
+    __shared__ __align__(16) float4 s_pos[GPB][NE | 1];
+    __shared__ __align__(16) float4 s_P[GPB][NQ * 3 | 1];
     __shared__ unsigned long long s_mbar;
     pdl_trigger();
-    stage_table(s_dN, gdN<E>(), NQ * NE * 3, &s_mbar, P.error);
-    pdl_wait();
-
     const int lane = threadIdx.x % G, grp = threadIdx.x / G;
     const XWork wk = work[blockIdx.x];   // GPB elements of one scene's colour
     const bool active = grp < wk.count;   // no early exit: every lane takes part in the shuffles
     const SceneDev& S = scenes[wk.scene];
-    const int eid = active ? S.elems[wk.begin + grp] : 0;   // for the quadrature records only
+    const int eid = active ? __ldg(S.elems + wk.begin + grp) : 0;   // for the quadrature records only
     const int* tp = S.etopo + (size_t)(active ? wk.begin + grp : 0) * NE;
     int vid[NI];
-    float4 u[NI];
     float w[NI];
-    bool mv[NI];
 #pragma unroll
     for (int k = 0; k < NI; ++k) {
         const int i = lane + k * G;
-        vid[k] = -1; u[k] = make_float4(0.f, 0.f, 0.f, 0.f); w[k] = 0.f; mv[k] = false;
-        if (active && i < NE) {
-            vid[k] = tp[i];
-            u[k] = S.u[vid[k]];
-            w[k] = 1.f / S.y[vid[k]].w;
-            mv[k] = RAW || S.mask[vid[k]] != 0;
-        }
+        vid[k] = active && i < NE ? __ldg(tp + i) : -1;
     }
+#pragma unroll
+    for (int k = 0; k < NI; ++k) w[k] = vid[k] >= 0 ? 1.f / S.y[vid[k]].w : 0.f;   // masses are static
     // quadrature record of lane q: JX_inv (columns m0 m1 m2), V, lambda, mu
     const int q = lane;
     const bool hasq = active && q < NQ;
@@ -1708,7 +1711,20 @@ __global__ void __launch_bounds__(kBlock, MINB) k_xpbd(const SceneDev* __restric
     const float4 L = active ? rec[2] : make_float4(0.f, 0.f, 1.f, 1.f);
     const float lam = L.z, mu = L.w;
     const float dt2 = P.dt * P.dt;
+    stage_table(s_dN, gdN<E>(), NQ * NE * 3, &s_mbar, P.error);
+    pdl_wait();
 
+    float4 u[NI];
+    bool mv[NI];
+#pragma unroll
+    for (int k = 0; k < NI; ++k) {
+        u[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        mv[k] = false;
+        if (vid[k] >= 0) {
+            u[k] = S.u[vid[k]];
+            mv[k] = RAW || S.mask[vid[k]] != 0;
+        }
+    }
     for (int m = 0; m < 2; ++m) {
 #pragma unroll
         for (int k = 0; k < NI; ++k)
@@ -1734,9 +1750,9 @@ __global__ void __launch_bounds__(kBlock, MINB) k_xpbd(const SceneDev* __restric
             // P~ = P JX_inv^T V: column j = sum_k P_k (m_k)_j
             const V3 T0 = (P0 * m0.x + P1 * m1.x + P2 * m2.x) * V, T1 = (P0 * m0.y + P1 * m1.y + P2 * m2.y) * V,
                      T2 = (P0 * m0.z + P1 * m1.z + P2 * m2.z) * V;
-            s_P[grp][q][0] = make_float4(T0.x, T0.y, T0.z, 0.f);
-            s_P[grp][q][1] = make_float4(T1.x, T1.y, T1.z, 0.f);
-            s_P[grp][q][2] = make_float4(T2.x, T2.y, T2.z, 0.f);
+            s_P[grp][3 * q] = make_float4(T0.x, T0.y, T0.z, 0.f);
+            s_P[grp][3 * q + 1] = make_float4(T1.x, T1.y, T1.z, 0.f);
+            s_P[grp][3 * q + 2] = make_float4(T2.x, T2.y, T2.z, 0.f);
         }
         float C = group_sum<G>(Cq);
         __syncwarp();
@@ -1750,24 +1766,36 @@ __global__ void __launch_bounds__(kBlock, MINB) k_xpbd(const SceneDev* __restric
 #pragma unroll
                 for (int qq = 0; qq < NQ; ++qq) {
                     const float* d = &s_dN[(qq * NE + i) * 3];
-                    const float4 a = s_P[grp][qq][0], b = s_P[grp][qq][1], c = s_P[grp][qq][2];
+                    const float4 a = s_P[grp][3 * qq], b = s_P[grp][3 * qq + 1], c = s_P[grp][3 * qq + 2];
                     g[k] = g[k] + mk(a.x, a.y, a.z) * d[0] + mk(b.x, b.y, b.z) * d[1] + mk(c.x, c.y, c.z) * d[2];
                 }
             }
         }
         const float k_st = m == 0 ? lam : mu;
         float step;
+        // P2's nodes are summed as by eight lanes (nodes 8 and 9 on the first two): the constraints
+        // are small differences, and another order changes a pass's last digits
         if (RAW) {
+            if constexpr (E == 7) {
+                ss = fmaf(dot(g[2], g[2]), w[2], __fmul_rn(dot(g[0], g[0]), w[0])) + __fmul_rn(dot(g[1], g[1]), w[1]);
+            } else {
 #pragma unroll
-            for (int k = 0; k < NI; ++k) ss += dot(g[k], g[k]) * w[k];
+                for (int k = 0; k < NI; ++k) ss += dot(g[k], g[k]) * w[k];
+            }
             const float S2 = group_sum<G>(ss);
             const float alpha = 4.f * C / (k_st * dt2);
             step = C < 1e-12f ? 0.f : -2.f * C / (S2 + alpha);
         } else {
             C = sqrtf(C < 0.f ? -C : C);
             const float ci = C < 1e-12f ? 0.f : 1.f / (2.f * C);
+            if constexpr (E == 7) {
 #pragma unroll
-            for (int k = 0; k < NI; ++k) { g[k] = g[k] * ci; ss += dot(g[k], g[k]) * w[k]; }
+                for (int k = 0; k < NI; ++k) g[k] = g[k] * ci;
+                ss = fmaf(dot(g[2], g[2]), w[2], __fmul_rn(dot(g[0], g[0]), w[0])) + __fmul_rn(dot(g[1], g[1]), w[1]);
+            } else {
+#pragma unroll
+                for (int k = 0; k < NI; ++k) { g[k] = g[k] * ci; ss += dot(g[k], g[k]) * w[k]; }
+            }
             const float S2 = group_sum<G>(ss);
             step = -C / (S2 + 1.f / (k_st * dt2));
         }
@@ -2383,12 +2411,12 @@ void vertex_mat(int mat, const SceneDev* scenes, const VWork* work, int n_work, 
 template <int E, bool RAW, int MINB>
 void xpbd_launch(int mat, const SceneDev* scenes, const XWork* work, int n_work, const StepParams& P, cudaStream_t st) {
     switch (mat) {
-        case 0: launch_pdl(k_xpbd<E, 0, RAW, MINB>, n_work, kBlock, 0, st, scenes, work, P); break;
-        case 1: launch_pdl(k_xpbd<E, 1, RAW, MINB>, n_work, kBlock, 0, st, scenes, work, P); break;
-        case 2: launch_pdl(k_xpbd<E, 2, RAW, MINB>, n_work, kBlock, 0, st, scenes, work, P); break;
-        case 3: launch_pdl(k_xpbd<E, 3, RAW, MINB>, n_work, kBlock, 0, st, scenes, work, P); break;
-        case 4: launch_pdl(k_xpbd<E, 4, RAW, MINB>, n_work, kBlock, 0, st, scenes, work, P); break;
-        default: launch_pdl(k_xpbd<E, 5, RAW, MINB>, n_work, kBlock, 0, st, scenes, work, P); break;
+        case 0: launch_pdl(k_xpbd<E, 0, RAW, MINB>, n_work, XpbdLanes<E>::kThreads, 0, st, scenes, work, P); break;
+        case 1: launch_pdl(k_xpbd<E, 1, RAW, MINB>, n_work, XpbdLanes<E>::kThreads, 0, st, scenes, work, P); break;
+        case 2: launch_pdl(k_xpbd<E, 2, RAW, MINB>, n_work, XpbdLanes<E>::kThreads, 0, st, scenes, work, P); break;
+        case 3: launch_pdl(k_xpbd<E, 3, RAW, MINB>, n_work, XpbdLanes<E>::kThreads, 0, st, scenes, work, P); break;
+        case 4: launch_pdl(k_xpbd<E, 4, RAW, MINB>, n_work, XpbdLanes<E>::kThreads, 0, st, scenes, work, P); break;
+        default: launch_pdl(k_xpbd<E, 5, RAW, MINB>, n_work, XpbdLanes<E>::kThreads, 0, st, scenes, work, P); break;
     }
 }
 template <int E, bool RAW>
@@ -2642,11 +2670,11 @@ int point_item_pairs(int element) { return element == 8 ? point_slots<8>() : poi
 
 int xpbd_elements_per_block(int element) {
     switch (element) {
-        case 3: return kBlock / XpbdLanes<3>::G;
-        case 6: return kBlock / XpbdLanes<6>::G;
-        case 7: return kBlock / XpbdLanes<7>::G;
-        case 8: return kBlock / XpbdLanes<8>::G;
-        case 9: return kBlock / XpbdLanes<9>::G;
+        case 3: return XpbdLanes<3>::kThreads / XpbdLanes<3>::G;
+        case 6: return XpbdLanes<6>::kThreads / XpbdLanes<6>::G;
+        case 7: return XpbdLanes<7>::kThreads / XpbdLanes<7>::G;
+        case 8: return XpbdLanes<8>::kThreads / XpbdLanes<8>::G;
+        case 9: return XpbdLanes<9>::kThreads / XpbdLanes<9>::G;
         default: return 1;
     }
 }
