@@ -153,7 +153,7 @@ class Scene:
         capi.check(capi.lib().oct_scene_sync(self._h), "oct_scene_sync", self.ctx.handle)
 
     def _get(self, fn):
-        out = np.zeros((self.n_nodes, 3), np.float32)
+        out = np.empty((self.n_nodes, 3), np.float32)
         capi.check(fn(self._h, capi.ptr(out, C.c_float)), fn.__name__, self.ctx.handle)
         return out
 
@@ -255,7 +255,7 @@ class Scene:
 
     def element_data(self, kind):
         """Per-element diagnostic (capi.DIAG_STRESS / VOLUME / VOLUME_DIFF / INVERTED)."""
-        out = np.zeros(self.n_elements, np.float32)
+        out = np.empty(self.n_elements, np.float32)
         capi.check(capi.lib().oct_scene_element_data(self._h, kind, capi.ptr(out, C.c_float)),
                    "oct_scene_element_data", self.ctx.handle)
         return out
