@@ -2197,13 +2197,34 @@ __global__ void __launch_bounds__(kBlock) k_element_diag(const SceneDev* __restr
     const double lam = c0.z, mu = c0.w;
     D3 A0 = {0, 0, 0}, A1 = A0, A2 = A0;   // accumulated Jx (kinds 4, 5, 6)
     double acc = 0.0;
-    for (int q = 0; q < NQ; ++q) {
-        D3 J0 = {0, 0, 0}, J1 = J0, J2 = J0, R0 = J0, R1 = J0, R2 = J0;
+    // The element's positions and rest positions, where they fit in registers, are gathered once
+    // and not once per point.
+    constexpr bool held = NE <= 10;
+    V3 pn[held ? NE : 1], xn[held ? NE : 1];
+    if constexpr (held) {
+#pragma unroll
         for (int i = 0; i < NE; ++i) {
             const int v = tp[i];
-            const float4 u = S.u[v], X = S.X[v];
-            const D3 p = {(double)(X.x + u.x), (double)(X.y + u.y), (double)(X.z + u.z)};
-            const D3 x = {(double)X.x, (double)X.y, (double)X.z};
+            const V3 u = xyz(S.u[v]);
+            xn[i] = xyz(S.X[v]);
+            pn[i] = xn[i] + u;
+        }
+    }
+#pragma unroll 1
+    for (int q = 0; q < NQ; ++q) {
+        D3 J0 = {0, 0, 0}, J1 = J0, J2 = J0, R0 = J0, R1 = J0, R2 = J0;
+#pragma unroll (held ? NE : 1)
+        for (int i = 0; i < NE; ++i) {
+            V3 pf, xf;
+            if constexpr (held) {
+                pf = pn[i]; xf = xn[i];
+            } else {
+                const int v = tp[i];
+                xf = xyz(S.X[v]);
+                pf = xf + xyz(S.u[v]);
+            }
+            const D3 p = {(double)pf.x, (double)pf.y, (double)pf.z};
+            const D3 x = {(double)xf.x, (double)xf.y, (double)xf.z};
             const double* d = dN + (q * NE + i) * 3;
             J0 = J0 + p * d[0]; J1 = J1 + p * d[1]; J2 = J2 + p * d[2];
             R0 = R0 + x * d[0]; R1 = R1 + x * d[1]; R2 = R2 + x * d[2];
@@ -2248,6 +2269,20 @@ void diag_launch(int mat, const SceneDev* scenes, int scene, int n_elements, int
 // ------------------------------------------------------------------------ FP64 energy
 // Kinetic + elastic + gravity energy of one scene in FP64 (new: the reference has no
 // energy evaluator; material energies of FEM_ContinuousMaterial.cpp:10-87).
+// Sum over a block of 256, in thread 0.  One FP64 atomic a block: with one a warp, 4,400 of them on
+// one word took most of the kernel (17 us for 140,481 nodes).
+__device__ __forceinline__ double block_sum(double v) {
+    __shared__ double part[8];
+    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+    __syncthreads();   // the last sum's parts have been read
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x != 0) return 0.0;
+    v = part[0];
+    for (int k = 1; k < (int)(blockDim.x >> 5); ++k) v += part[k];
+    return v;
+}
+
 template <int E>
 __global__ void k_energy_elements(const SceneDev* __restrict__ scenes, int scene, int material, double* out, int* error) {
     constexpr int NE = ElemT<E>::NE, NQ = ElemT<E>::NQ;
@@ -2256,12 +2291,20 @@ __global__ void k_energy_elements(const SceneDev* __restrict__ scenes, int scene
     for (int eid = blockIdx.x * blockDim.x + threadIdx.x; eid < S.n_elements; eid += gridDim.x * blockDim.x) {
         const int* tp = S.topo + (size_t)eid * NE;
         const float* cd = cdN<E>();
+        constexpr bool held = NE <= 10;   // the element's nodes fit in registers: gathered once
+        V3 un[held ? NE : 1];
+        if constexpr (held) {
+#pragma unroll
+            for (int i = 0; i < NE; ++i) un[i] = xyz(S.u[tp[i]]);
+        }
+#pragma unroll 1
         for (int q = 0; q < NQ; ++q) {
             const size_t ri = ((size_t)eid * S.eq_stride + (S.eq_stride == 1 ? 0 : q)) * 3;
             const float4 A = S.eq[ri], B = S.eq[ri + 1], C = S.eq[ri + 2];
             double J[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};   // J[col][row]
+#pragma unroll (held ? NE : 1)
             for (int i = 0; i < NE; ++i) {
-                const float4 u = S.u[tp[i]];
+                const V3 u = held ? un[held ? i : 0] : xyz(S.u[tp[i]]);
                 for (int c = 0; c < 3; ++c) {
                     const double d = cd[(q * NE + i) * 3 + c];
                     J[c][0] += (double)u.x * d; J[c][1] += (double)u.y * d; J[c][2] += (double)u.z * d;
@@ -2300,8 +2343,8 @@ __global__ void k_energy_elements(const SceneDev* __restrict__ scenes, int scene
         }
     }
     if (!isfinite(local)) atomicOr(error, 2);
-    for (int off = 16; off > 0; off >>= 1) local += __shfl_xor_sync(0xffffffffu, local, off);
-    if ((threadIdx.x & 31) == 0) atomicAdd(out + 1, local);
+    local = block_sum(local);
+    if (threadIdx.x == 0) atomicAdd(out + 1, local);
 }
 
 __global__ void k_energy_nodes(const SceneDev* __restrict__ scenes, int scene, double* out, int* error) {
@@ -2315,11 +2358,9 @@ __global__ void k_energy_nodes(const SceneDev* __restrict__ scenes, int scene, d
         grav -= m * (S.gx * px + S.gy * py + S.gz * pz);
     }
     if (!isfinite(kin) || !isfinite(grav)) atomicOr(error, 2);
-    for (int off = 16; off > 0; off >>= 1) {
-        kin += __shfl_xor_sync(0xffffffffu, kin, off);
-        grav += __shfl_xor_sync(0xffffffffu, grav, off);
-    }
-    if ((threadIdx.x & 31) == 0) { atomicAdd(out + 0, kin); atomicAdd(out + 2, grav); }
+    kin = block_sum(kin);
+    grav = block_sum(grav);
+    if (threadIdx.x == 0) { atomicAdd(out + 0, kin); atomicAdd(out + 2, grav); }
 }
 
 // ------------------------------------------------------------------------ launchers
