@@ -1228,10 +1228,10 @@ struct GridBarrier {
     __device__ __forceinline__ bool wait(int* error) {
         if (gridDim.x > 1 && threadIdx.x == 0) {
             unsigned seen = 0;
-            int it = 0;
+            long it = 0;
             do {
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
-            } while ((int)(seen - target) < 0 && ++it < (1 << 20));
+            } while ((int)(seen - target) < 0 && ++it < kSpinLimit);
             if ((int)(seen - target) < 0) { atomicOr(error, 1); alive = false; }
         }
         return !__syncthreads_or(threadIdx.x == 0 && !alive);
