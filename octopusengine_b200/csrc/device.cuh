@@ -15,7 +15,7 @@
 // instead of NQ), which divides the per-visit element bytes by NQ.  The inverse reference
 // Jacobians are computed in FP64 on the host and rounded once.
 //
-// Colour-sorted vertex slots: vids[slot] is the node solved in that slot; slots of colour
+// Colour-sorted vertex slots: slots[slot].x is the node solved in that slot; slots of colour
 // c are [color_off[c], color_off[c+1]) in ascending node id (GPU_VBD_FEM::create_buffers,
 // octopus/src/GPU/VBD/GPU_VBD_FEM.cu:594-675); owners is the owner CSR in slot order
 // (slots holds each slot's part of it) with owners packed as (element id << 5) | local node index.
@@ -60,12 +60,11 @@ struct SceneDev {
     const float4* X;    // rest positions
     const int* topo;    // n_elements * NE
     const float4* eq;   // n_elements * NQ * 3
-    const int* vids;    // n_nodes, colour-sorted
-    const int4* slots;  // the same slots with their owners: node, first owner, owner count, 0
+    const int4* slots;  // n_nodes, colour-sorted: node, first owner, owner count, 0
     const int* owners;  // packed (eid << 5) | r
     const int* fixed;   // n_fixed node ids
     const int* fixed_group;            // n_fixed rigid-group indices
-    const int* fix_of;                 // VBD, explicit: per node its rigid group if fixed, else -1 (or null)
+    const int* fix_of;                 // explicit, VBD with Chebyshev: per node its rigid group if fixed, else -1 (or null)
     const int* topo_t;                 // explicit: the topology node by node, [local node][element]
     const int* owner_at;               // explicit: place of (element, local node) in owners, [local node][element]
     const float* fix;                  // kFixGroups x 16: com (3), offset (3), rotation (9, column-major), pad

@@ -1516,7 +1516,7 @@ __global__ void k_commit(const SceneDev* __restrict__ scenes, const VWork* __res
         const VWork wk = work[w];
         const SceneDev& S = scenes[wk.scene];
         for (int k = threadIdx.x; k < wk.count; k += blockDim.x) {
-            const int vid = S.vids[wk.slot_begin + k];
+            const int vid = S.slots[wk.slot_begin + k].x;
             if (S.mask[vid] != 0) S.u[vid] = S.u_new[vid];
         }
     }

@@ -900,10 +900,10 @@ oct_status build_scene(oct_ctx* c, const oct_scene_desc* d, oct_scene* s) {
     if (s->rho > 0.f) {
         if ((st = upload(c, s->mem, p1, zero4)) || (st = upload(c, s->mem, p2, zero4))) return st;
     }
-    int *maskd, *topod, *vidsd, *ownd, *fixd = nullptr;
+    int *maskd, *topod, *ownd, *fixd = nullptr;
     float4* eqd;
     if ((st = upload(c, s->mem, maskd, mask)) || (st = upload(c, s->mem, topod, topo)) || (st = upload(c, s->mem, eqd, eq)) ||
-        (st = upload(c, s->mem, vidsd, slot_vids)) || (st = upload(c, s->mem, ownd, owners)))
+        (st = upload(c, s->mem, ownd, owners)))
         return st;
     std::vector<int4> slots(N);
     for (int sl = 0; sl < N; ++sl) slots[sl] = make_int4(slot_vids[sl], own_off[sl], own_off[sl + 1] - own_off[sl], 0);
@@ -914,9 +914,9 @@ oct_status build_scene(oct_ctx* c, const oct_scene_desc* d, oct_scene* s) {
     if (s->n_fixed && ((st = upload(c, s->mem, fixd, s->fixed)) || (st = upload(c, s->mem, fgd, s->fixed_group)))) return st;
     if ((st = upload(c, s->mem, s->d_fix, std::vector<float>(s->fix_host, s->fix_host + kFixGroups * 16)))) return st;
     h.u = u; h.u_last = ul; h.y = y; h.v = v; h.u_new = un; h.prev1 = p1; h.prev2 = p2; h.mask = maskd; h.X = Xd;
-    h.topo = topod; h.eq = eqd; h.vids = vidsd; h.owners = ownd; h.fixed = fixd;
+    h.topo = topod; h.eq = eqd; h.owners = ownd; h.fixed = fixd;
     h.fixed_group = fgd; h.fix = s->d_fix;
-    if (d->solver != OCT_SOLVER_XPBD && s->n_fixed) {   // for the updates that apply the fixation node by node
+    if (s->n_fixed && (d->solver == OCT_SOLVER_EXPLICIT || (d->solver == OCT_SOLVER_VBD && s->rho > 0.f))) {   // updates that apply the fixation node by node
         std::vector<int32_t> fix_of(N, -1);
         for (int k = 0; k < s->n_fixed; ++k) fix_of[s->fixed[k]] = s->fixed_group[k];
         int* fod;
@@ -946,7 +946,7 @@ oct_status build_scene(oct_ctx* c, const oct_scene_desc* d, oct_scene* s) {
     // records than the P1 entry can index) the colour kernels read owners, topology and records
     h.ent = nullptr;
     h.rtab = nullptr;
-    if ((int64_t)N <= (int64_t)kIdMask + 1) {
+    if (d->solver == OCT_SOLVER_VBD && (int64_t)N <= (int64_t)kIdMask + 1) {   // read by the VBD kernels only
         const int EW = entry_words(NE);
         const bool affine = h.eq_stride == 1;
         // distinct records, compared bit for bit (identical records give identical results)
@@ -1028,7 +1028,7 @@ oct_status build_scene(oct_ctx* c, const oct_scene_desc* d, oct_scene* s) {
             s->n_records = (int64_t)rtab.size() / 3;
         }
     }
-    if (!h.ent && s->tpv == 0) s->tpv = default_tpv(d->element);   // the packed mapping streams entries
+    if (d->solver == OCT_SOLVER_VBD && !h.ent && s->tpv == 0) s->tpv = default_tpv(d->element);   // the packed mapping streams entries
     for (int k = 0; k < kMaxEffects; ++k) { s->effects[k] = EffectDev{}; s->effects[k].kind = -1; }
     if ((st = upload(c, s->mem, s->d_effects, std::vector<EffectDev>(s->effects, s->effects + kMaxEffects)))) return st;
     h.effects = s->d_effects;
@@ -1044,8 +1044,8 @@ oct_status build_scene(oct_ctx* c, const oct_scene_desc* d, oct_scene* s) {
     // predictor; XPBD and explicit step the velocity array itself, which already holds it
     s->pending_host = s->has_v0 && d->solver == OCT_SOLVER_VBD ? 1 : 0;
     if ((st = upload(c, s->mem, s->d_pending, std::vector<int>{s->pending_host}))) return st;
-    if ((st = s->mem.alloc(s->d_red, 4))) return st;
-    if ((st = upload(c, s->mem, s->d_bar, std::vector<unsigned>(2, 0u)))) return st;
+    if ((st = upload(c, s->mem, s->d_red, std::vector<double>(5, 0.0)))) return st;
+    s->d_bar = reinterpret_cast<unsigned*>(s->d_red + 4);
     if (d->solver == OCT_SOLVER_EXPLICIT && (st = s->mem.alloc(s->d_contrib, (size_t)E * NE))) return st;
 
     // work tables
@@ -2171,7 +2171,7 @@ oct_status oct_scene_set_mapping(oct_scene* s, int tpv) {
         if (tpv < 0) return fail(s->ctx, OCT_ENOTSUP, "packed mapping needs at most 32 owners per vertex");
         t = s->max_valence > 64 ? 32 : default_tpv(s->element);
     }
-    if (t == 0 && !s->h.ent) {
+    if (t == 0 && s->solver == OCT_SOLVER_VBD && !s->h.ent) {
         if (tpv < 0) return fail(s->ctx, OCT_ENOTSUP, "packed mapping needs owner entries (scene past their index range)");
         t = default_tpv(s->element);
     }
