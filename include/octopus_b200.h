@@ -416,6 +416,11 @@ oct_status oct_scene_restore(oct_scene* s, const float* in);
  * that never completes, with at most limit (<= 1e6) polls, and returns OCT_ETIMEDOUT through
  * the context's error word; the context stays usable. */
 oct_status oct_ctx_wait_probe(oct_ctx* ctx, int32_t limit);
+/* The same for the grid barrier of the scene's one-launch sub-step: a small grid waits, with at
+ * most limit (<= 1e6) looks, for an arrival that never comes.  Returns OCT_ETIMEDOUT; the scene's
+ * own status (oct_scene_status) reports it too, whoever reads the context's word first, and the
+ * scene can be stepped again. */
+oct_status oct_scene_wait_probe(oct_scene* s, int32_t limit);
 
 /* Measurement helpers.  The context's CUDA stream (cudaStream_t), to record events on it. */
 oct_status oct_ctx_stream(oct_ctx* ctx, void** stream);

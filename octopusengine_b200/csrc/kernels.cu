@@ -1216,30 +1216,52 @@ __global__ void k_constraints(const SceneDev* __restrict__ scenes, const NWork* 
 // empties L1.
 constexpr int kSubBlocks = 4;
 
-// Barrier over the grid: bar[0] counts arrivals.  The wait has an iteration limit; a block that
-// gives up records the time-out and returns false, and so do the others that it leaves waiting.
+// Barrier over the grid: bar[0] counts arrivals, bar[1] blocks that have left.  The wait has an
+// iteration limit; a block that gives up records the time-out, in the context's word and in the
+// scene's (the scene's sub-step is left half done), and returns false, and so do the others that it
+// leaves waiting.
 struct GridBarrier {
     unsigned* bar;
+    int* error;
+    int* status;
+    long limit;
     unsigned target;
     bool alive;
-    __device__ __forceinline__ void arrive() {
+    __device__ __forceinline__ void arrive(bool counted = true) {
         __syncthreads();
         if (gridDim.x == 1) return;
         target += gridDim.x;
-        if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+        if (threadIdx.x == 0 && counted) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
     }
-    __device__ __forceinline__ bool wait(int* error) {
+    __device__ __forceinline__ bool wait() {
         if (gridDim.x > 1 && threadIdx.x == 0) {
             unsigned seen = 0;
             long it = 0;
             do {
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
-            } while ((int)(seen - target) < 0 && ++it < kSpinLimit);
-            if ((int)(seen - target) < 0) { atomicOr(error, 1); alive = false; }
+            } while ((int)(seen - target) < 0 && ++it < limit);
+            if ((int)(seen - target) < 0) { atomicOr(error, 1); atomicOr(status, kStatusTimeout); alive = false; }
         }
         return !__syncthreads_or(threadIdx.x == 0 && !alive);
     }
+    // Every block has left its last barrier, or given it up, once it counts itself here: the last one
+    // clears both words for the next launch.
+    __device__ __forceinline__ void leave() {
+        if (threadIdx.x != 0 || gridDim.x == 1) return;
+        unsigned before;
+        asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(bar + 1) : "memory");
+        if (before == gridDim.x - 1) { bar[0] = 0u; bar[1] = 0u; }
+    }
 };
+
+// Failure-detection probe: a grid barrier at which the first block does not arrive, so every block
+// of the grid gives up after `limit` looks.
+__global__ void k_barrier_probe(unsigned* bar, int* error, int* status, long limit) {
+    GridBarrier gb{bar, error, status, limit, 0u, true};
+    gb.arrive(blockIdx.x != 0);
+    gb.wait();
+    gb.leave();
+}
 
 template <int E, int MAT>
 __global__ void __launch_bounds__(kSubBlocks * kBlock, 1)
@@ -1278,14 +1300,14 @@ k_vbd_substep(const SceneDev* __restrict__ scene, const VWork* __restrict__ work
             for (int j = 0; j < EW / 4; ++j) nxt[j] = ld_hint(S.ent + (size_t)o * (EW / 4) + j, stream);
         }
     };
-    GridBarrier gb{bar, 0u, true};
+    GridBarrier gb{bar, P.error, S.status, kSpinLimit, 0u, true};
     bool alive = true;
     const bool pending = P.pending_v0 && *P.pending_v0;
     for (int i = node0; i < S.n_nodes; i += nodes) vbd_predict(S, i, pending, cheb, P.dt, P.inv_dt);
     int c_begin = __ldg(colour_off), c_end = __ldg(colour_off + 1);
     gb.arrive();
     fetch(c_begin + first, c_end);
-    alive = gb.wait(P.error);
+    alive = gb.wait();
     float omega = 1.f;
     for (int j = 0; j < iterations && alive; ++j) {
         for (int c = 0; c < n_colours && alive; ++c) {
@@ -1328,7 +1350,7 @@ k_vbd_substep(const SceneDev* __restrict__ scene, const VWork* __restrict__ work
             c_end = __ldg(colour_off + next + 1);
             gb.arrive();
             fetch(c_begin + first, c_end);
-            alive = gb.wait(P.error);
+            alive = gb.wait();
         }
         const bool fix = j == 0 && S.n_fixed > 0;
         if (alive && (fix || cheb)) {
@@ -1343,13 +1365,12 @@ k_vbd_substep(const SceneDev* __restrict__ scene, const VWork* __restrict__ work
                 for (int k = node0; k < S.n_fixed; k += nodes) fix_node(S, S.fixed[k], S.fixed_group[k]);
             }
             gb.arrive();
-            alive = gb.wait(P.error);
+            alive = gb.wait();
         }
     }
     if (alive)
         for (int i = node0; i < S.n_nodes; i += nodes) vbd_velocity(S, i, P.dt);
-    // every block has left its last barrier once it counts itself here: the last one clears both
-    if (threadIdx.x == 0 && gridDim.x > 1 && atomicAdd(bar + 1, 1u) == gridDim.x - 1) { bar[0] = 0u; bar[1] = 0u; }
+    gb.leave();
 }
 
 // Scripted effects (GPU_Constraint.cu:22-92), run after the fixation in creation order.
@@ -2647,6 +2668,11 @@ void launch_mg_prolong(const SceneDev* main, const int* list, int count, int k, 
 }
 
 void launch_wait_probe(int* error, long limit, cudaStream_t st) { k_wait_probe<<<1, 1, 0, st>>>(error, limit); }
+
+bool launch_barrier_probe(unsigned* bar, int* error, int* status, long limit, cudaStream_t st) {
+    void* args[] = {&bar, &error, &status, &limit};
+    return cudaLaunchCooperativeKernel(k_barrier_probe, dim3(4), dim3(64), args, 0, st) == cudaSuccess;
+}
 void launch_nodes_out(const float4* src, const float4* X, float* out, int n, cudaStream_t st) {
     if (n > 0) k_nodes_out<<<(n + 255) / 256, 256, 0, st>>>(src, X, out, n);
 }

@@ -46,6 +46,9 @@ void launch_nodes_out(const float4* src, const float4* X, float* out, int n, cud
 void launch_nodes_in(const float* in, const float4* X, float4* dst, int n, cudaStream_t st);
 // Failure-detection probe: a bounded wait on a phase nothing completes (error bit 0 on time-out).
 void launch_wait_probe(int* error, long limit, cudaStream_t st);
+// The same for the grid barrier of the one-launch sub-step: one arrival fewer than the barrier
+// waits for (error bit 0 and kStatusTimeout in status; bar is left zeroed).
+bool launch_barrier_probe(unsigned* bar, int* error, int* status, long limit, cudaStream_t st);
 // One scripted effect of one scene (kind 0 crush / 1 random sphere over the node chunks in
 // work, kind 2 high stretch over its ids); a no-op while the effect is inactive.
 void launch_effect(const SceneDev* scene, const NWork* work, int n_work, int slot, int kind, float dt, cudaStream_t st);

@@ -1632,6 +1632,17 @@ oct_status oct_ctx_wait_probe(oct_ctx* c, int32_t limit) {
     return sync_and_check(c);
 }
 
+oct_status oct_scene_wait_probe(oct_scene* s, int32_t limit) {
+    if (!s || limit <= 0 || limit > 1000000) return OCT_EINVAL;
+    oct_ctx* c = s->ctx;
+    unsigned left[2] = {1u, 1u};
+    if (!launch_barrier_probe(s->d_bar, c->d_error, s->d_status, limit, c->stream)) OCT_CUDA(c, cudaGetLastError());
+    OCT_CUDA(c, cudaStreamSynchronize(c->stream));
+    OCT_CUDA(c, cudaMemcpy(left, s->d_bar, sizeof(left), cudaMemcpyDeviceToHost));
+    if (left[0] || left[1]) return fail(c, OCT_ECUDA, "the grid barrier's words are not zero after a time-out");
+    return sync_and_check(c);
+}
+
 // Checkpoint: per node u, u_last, v (9 floats) and the mask, then the fixation table
 // (kFixGroups x 16), the effects' stretch distances (kMaxEffects), the multigrid schedule (3)
 // and the pending initial-velocity flag.
