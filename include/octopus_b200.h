@@ -421,6 +421,9 @@ oct_status oct_ctx_wait_probe(oct_ctx* ctx, int32_t limit);
  * own status (oct_scene_status) reports it too, whoever reads the context's word first, and the
  * scene can be stepped again. */
 oct_status oct_scene_wait_probe(oct_scene* s, int32_t limit);
+/* The context's next n cooperative launches are taken as refused by the driver, on the host: each
+ * scene that meets one runs its sub-steps with a launch per colour from then on (the same bits). */
+oct_status oct_ctx_refuse_probe(oct_ctx* ctx, int32_t n);
 
 /* Measurement helpers.  The context's CUDA stream (cudaStream_t), to record events on it. */
 oct_status oct_ctx_stream(oct_ctx* ctx, void** stream);

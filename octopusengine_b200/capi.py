@@ -48,7 +48,7 @@ EXPORTS = [
     "oct_beam_sampler_error", "oct_beam_sampler_destroy", "oct_flexion_error", "oct_torsion_profile",
     "oct_scene_add_effect", "oct_scene_set_effect_active", "oct_scene_effect_ids", "oct_surface_nodes",
     "oct_scene_state_size", "oct_scene_save", "oct_scene_restore", "oct_ctx_wait_probe",
-    "oct_scene_wait_probe",
+    "oct_scene_wait_probe", "oct_ctx_refuse_probe",
     "oct_scene_status", "oct_batch_status",
 ]
 
@@ -139,6 +139,7 @@ def lib():
             "oct_scene_restore": ([vp, C.POINTER(C.c_float)], C.c_int),
             "oct_ctx_wait_probe": ([vp, C.c_int32], C.c_int),
             "oct_scene_wait_probe": ([vp, C.c_int32], C.c_int),
+            "oct_ctx_refuse_probe": ([vp, C.c_int32], C.c_int),
             "oct_scene_set_effect_active": ([vp, C.c_int32, C.c_int], C.c_int),
             "oct_scene_effect_ids": ([vp, C.c_int32, C.POINTER(C.c_int32), C.POINTER(C.c_int32)], C.c_int),
             "oct_surface_nodes": ([C.c_int32, C.POINTER(C.c_int32), C.c_int32, C.POINTER(C.c_int32), C.POINTER(C.c_int32)],

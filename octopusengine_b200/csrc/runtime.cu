@@ -129,6 +129,7 @@ struct oct_ctx {
     uint64_t launches = 0;
     bool tables[10] = {false};
     int sms = 0;         // streaming multiprocessors (sm_count)
+    int refuse = 0;      // oct_ctx_refuse_probe: cooperative launches still to be taken as refused
     std::mutex mu;       // guards the budget accounting and the shape-table upload
     std::mutex err_mu;   // guards err (scenes may be created from several host threads)
     // device blocks released by destroyed scenes and batches, kept for reuse (size -> pointer):
@@ -255,6 +256,7 @@ struct oct_scene {
     int* d_vwork_off = nullptr;
     int max_items = 0;              // most work items of a colour
     unsigned* d_bar = nullptr;      // grid barrier of the one-launch sub-step
+    bool one_launch_refused = false;   // the driver refused its cooperative launch: a launch per colour from then on
     NWork* d_nwork = nullptr;
     int n_nwork = 0;
     NWork* d_fwork = nullptr;
@@ -1099,7 +1101,7 @@ int sm_count(oct_ctx* c) {
 // 2,025 nodes 3.3 / 4.5, 40,625 nodes 4.4 / 5.5; P2 140,481 nodes, 308 items, a frame of five
 // sub-steps 4.56 / 4.38 ms).
 bool one_launch(const oct_scene* s) {
-    return s->max_items <= 2 * sm_count(s->ctx) && s->tpv > 0 && (s->element == kTetra || s->element == kHexa || s->element == kTetra10) && s->h.ent &&
+    return !s->one_launch_refused && s->max_items <= 2 * sm_count(s->ctx) && s->tpv > 0 && (s->element == kTetra || s->element == kHexa || s->element == kTetra10) && s->h.ent &&
            s->in_place && s->order_mode == OCT_ORDER_ASCENDING && !s->mg_sub && !s->n_effects && !s->box;
 }
 
@@ -1129,11 +1131,16 @@ void vbd_substep(oct_scene* s, float dt) {
     if (one_launch(s)) {
         const int sms = sm_count(c);
         const int grid = s->max_items <= 2 * kSubBlocks ? 1 : std::min(s->max_items, sms);
-        launch_vbd_substep(s->element, s->material, s->d_scene, s->d_vwork, s->d_vwork_off, s->n_colors, s->iterations,
-                           cheb ? s->rho : 0.f, s->d_bar, grid, P, st);
-        c->launches++;
-        consumed();
-        return;
+        const bool taken = c->refuse > 0 ? (--c->refuse, false) :
+            launch_vbd_substep(s->element, s->material, s->d_scene, s->d_vwork, s->d_vwork_off, s->n_colors, s->iterations,
+                               cheb ? s->rho : 0.f, s->d_bar, grid, P, st);
+        if (taken) {
+            c->launches++;
+            consumed();
+            return;
+        }
+        cudaGetLastError();   // fewer co-resident blocks than SMs (a partitioned device): the same work, a launch per colour
+        s->one_launch_refused = true;
     }
     launch_predict(s->d_scene, s->d_nwork, s->n_nwork, 0, 0, cheb ? 1 : 0, P, st);
     c->launches++;
@@ -1403,7 +1410,11 @@ oct_status oct_scene_step(oct_scene* s, float frame_dt, int substeps) {
         const cudaError_t e = cudaStreamEndCapture(c->stream, &g);
         s->frame_launches = c->launches - l0;
         c->launches = l0;
-        if (e != cudaSuccess) return fail(c, OCT_ECUDA, std::string("frame capture: ") + cudaGetErrorString(e));
+        const cudaError_t el = cudaGetLastError();   // of a launch that the graph would lack
+        if (e != cudaSuccess || el != cudaSuccess) {
+            if (g) cudaGraphDestroy(g);
+            return fail(c, OCT_ECUDA, std::string("frame capture: ") + cudaGetErrorString(e != cudaSuccess ? e : el));
+        }
         const cudaError_t ei = cudaGraphInstantiate(&s->frame_exec, g, 0);
         cudaGraphDestroy(g);
         if (ei != cudaSuccess) {
@@ -1630,6 +1641,12 @@ oct_status oct_ctx_wait_probe(oct_ctx* c, int32_t limit) {
     launch_wait_probe(c->d_error, limit, c->stream);
     OCT_CUDA(c, cudaGetLastError());
     return sync_and_check(c);
+}
+
+oct_status oct_ctx_refuse_probe(oct_ctx* c, int32_t n) {
+    if (!c || n < 0) return OCT_EINVAL;
+    c->refuse = n;
+    return OCT_OK;
 }
 
 oct_status oct_scene_wait_probe(oct_scene* s, int32_t limit) {

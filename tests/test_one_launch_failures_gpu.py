@@ -1,5 +1,6 @@
 """Failures of the one-launch VBD sub-step, without faulting the GPU: a grid barrier that runs out
-of looks is reported by the scene it belongs to and leaves the scene usable."""
+of looks is reported by the scene it belongs to and leaves the scene usable; a cooperative launch
+that the driver refuses is replaced by the launches per colour, also in a captured frame."""
 import numpy as np
 import pytest
 
@@ -27,3 +28,28 @@ def test_a_barrier_time_out_belongs_to_its_scene(ctx, element):
     check_parity(s.get_position(), o32, o64, mesh["X"], "e%d" % element)
     np.testing.assert_array_equal(s.get_position(), other.get_position())
     assert s.status() == 0
+
+
+@pytest.mark.parametrize("capture", [False, True])
+@pytest.mark.parametrize("element,cells", [(O.TETRA, (1, 1, 1)), (O.HEXA, (12, 5, 4)), (O.TETRA10, (6, 3, 3))])
+def test_a_refused_launch_falls_back_to_launches_per_colour(ctx, element, cells, capture):
+    from octopusengine_b200 import capi
+    X, _ = O.beam_mesh(element, cells, tuple(0.125 * c for c in cells))
+    v0 = np.random.default_rng(1).normal(0.0, 0.05, X.shape).astype(np.float32)   # a pending first velocity
+    kw = dict(cells=cells, size=tuple(0.125 * c for c in cells), iterations=4, rho=0.9, v0=v0)
+    s, twin = pair(ctx, element, **kw)[0], pair(ctx, element, **kw)[0]
+    s.set_capture(capture)
+    twin.set_capture(capture)
+    twin.step(1 / 60, 2)
+    assert capi.lib().oct_ctx_refuse_probe(ctx.handle, 0 if capture else 1) == 0
+    s.step(1 / 60, 2)
+    if capture:   # the first frame, with the pending velocity, is not captured
+        assert capi.lib().oct_ctx_refuse_probe(ctx.handle, 1) == 0
+    for _ in range(3):   # the frame that meets the refusal, and replays of it
+        s.step(1 / 60, 2)
+    assert capi.lib().oct_ctx_refuse_probe(ctx.handle, 0) == 0
+    for _ in range(3):
+        twin.step(1 / 60, 2)
+    np.testing.assert_array_equal(s.get_position(), twin.get_position())
+    np.testing.assert_array_equal(s.get_velocity(), twin.get_velocity())
+    assert np.abs(s.get_velocity()).max() > 0
