@@ -183,6 +183,12 @@ __device__ __forceinline__ V3 operator-(V3 a, V3 b) { return {a.x - b.x, a.y - b
 __device__ __forceinline__ V3 operator*(V3 a, float s) { return {a.x * s, a.y * s, a.z * s}; }
 __device__ __forceinline__ float dot(V3 a, V3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
 __device__ __forceinline__ V3 cross(V3 a, V3 b) { return {a.y * b.z - b.y * a.z, a.z * b.x - b.z * a.x, a.x * b.y - b.x * a.y}; }
+// A column of F's cofactor.  The subtracted product is the rounded one: near the identity the other
+// is, in the entry that counts, a product of two diagonal entries, and rounding it as well would add
+// the result's largest error (left to the compiler, that differs from kernel to kernel).
+__device__ __forceinline__ V3 cofactor(V3 a, V3 b) {
+    return {fmaf(a.y, b.z, -(b.y * a.z)), fmaf(a.z, b.x, -(b.z * a.x)), fmaf(a.x, b.y, -(b.x * a.y))};
+}
 __device__ __forceinline__ V3 xyz(float4 a) { return {a.x, a.y, a.z}; }
 
 // Compensated accumulation (Kahan): s + c carries the running sum to ~2^-48 relative.
@@ -210,11 +216,12 @@ __device__ __forceinline__ void material_terms(V3 F0, V3 F1, V3 F2, V3 g, float 
     const float gg = dot(g, g);
     const V3 a = F0 * g.x + F1 * g.y + F2 * g.z;   // F g
     if (MAT == 2 || MAT == 3) {
-        const V3 C0 = cross(F1, F2), C1 = cross(F2, F0), C2 = cross(F0, F1);
-        const float J = dot(F0, C0);
+        const V3 C0 = cofactor(F1, F2), C1 = cofactor(F2, F0), C2 = cofactor(F0, F1);
+        // J - 1 without a rounding near one: lambda multiplies what that leaves
+        const float J1 = fmaf(F0.x, C0.x, -1.f) + fmaf(F0.y, C0.y, F0.z * C0.z);
         const V3 h = C0 * g.x + C1 * g.y + C2 * g.z;   // cof(F) g
         // lambda (J - alpha) with alpha = 1 + mu/lambda (Stable NH) or 1 (NH)
-        const float s = MAT == 3 ? lam * (J - 1.f) - mu : lam * (J - 1.f);
+        const float s = MAT == 3 ? lam * J1 - mu : lam * J1;
         const V3 Pg = a * mu + h * s;
         const float lv = lam * V, dv = mu * gg * V;
         out[0] = -V * Pg.x; out[1] = -V * Pg.y; out[2] = -V * Pg.z;
@@ -715,8 +722,11 @@ template <int E> constexpr int packed_smem_bytes() { return (kBlock / 32) * 2 * 
 // pair, three points each (P3 4 lanes, Q2 9), so a launch has LP times the lanes and a chain a
 // quarter to a ninth as long, for the same work per pair or less:
 //   Q2: the lane's three points share (y, z), and the basis is a tensor product, so the node
-//       displacements are contracted along z, then y (18 + 9 values per column of nodes), then
-//       along x at the three points: 324 FMAs where three dense contractions took 729;
+//       displacements are contracted along z, then y, then along x at the three points, a third of
+//       the operations of three dense contractions.  Along each direction the 1-D basis sums to one
+//       and its derivative to zero, so both act on the differences to the middle node: as many
+//       operations as the three products, and the rounding of the basis values no longer meets the
+//       displacement itself (force error of a smooth pose 12.5 -> 11.0 units of 2^-24);
 //   P3: the dense contraction per point, its dN row read from shared memory.
 // A pair's nodes are gathered once by its lanes into shared memory.  A block takes whole vertices
 // up to its number of pair slots; a pair's lanes are summed first, then each vertex's pairs in
@@ -784,15 +794,16 @@ k_vertex_points(const SceneDev* __restrict__ scenes, const VWork* __restrict__ w
     };
     int w = blockIdx.x;
     fetch(w);
-    [[maybe_unused]] float ny[3], dy[3], nz[3], dz[3];   // Q2: the lane's basis values along y and z
+    // Q2: the lane's basis values along y and z, of the outer nodes
+    [[maybe_unused]] float ny[2], dy[2], nz[2], dz[2];
     if constexpr (E == 9) {
         const int b = j % 3, c = j / 3;
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            ny[k] = b == 0 ? q2_n(0, k) : b == 1 ? q2_n(1, k) : q2_n(2, k);
-            dy[k] = b == 0 ? q2_d(0, k) : b == 1 ? q2_d(1, k) : q2_d(2, k);
-            nz[k] = c == 0 ? q2_n(0, k) : c == 1 ? q2_n(1, k) : q2_n(2, k);
-            dz[k] = c == 0 ? q2_d(0, k) : c == 1 ? q2_d(1, k) : q2_d(2, k);
+        for (int k = 0; k < 2; ++k) {
+            ny[k] = b == 0 ? q2_n(0, 2 * k) : b == 1 ? q2_n(1, 2 * k) : q2_n(2, 2 * k);
+            dy[k] = b == 0 ? q2_d(0, 2 * k) : b == 1 ? q2_d(1, 2 * k) : q2_d(2, 2 * k);
+            nz[k] = c == 0 ? q2_n(0, 2 * k) : c == 1 ? q2_n(1, 2 * k) : q2_n(2, 2 * k);
+            dz[k] = c == 0 ? q2_d(0, 2 * k) : c == 1 ? q2_d(1, 2 * k) : q2_d(2, 2 * k);
         }
     }
     [[maybe_unused]] int qs[PP];   // Q2: the lane's points (x = a) and their weights
@@ -843,14 +854,19 @@ k_vertex_points(const SceneDev* __restrict__ scenes, const VWork* __restrict__ w
                 if constexpr (E == 9) {
 #pragma unroll
                     for (int a = 0; a < 3; ++a) {
-                        cv[a] = cy[a] = cz[a] = mk(0.f, 0.f, 0.f);
+                        V3 v[3], d[3];
 #pragma unroll
                         for (int b = 0; b < 3; ++b) {
                             const V3 u0 = xyz(s_u[slot][q2_index(a, b, 0)]), u1 = xyz(s_u[slot][q2_index(a, b, 1)]),
                                      u2 = xyz(s_u[slot][q2_index(a, b, 2)]);
-                            const V3 v = u0 * nz[0] + u1 * nz[1] + u2 * nz[2], d = u0 * dz[0] + u1 * dz[1] + u2 * dz[2];
-                            cv[a] = cv[a] + v * ny[b]; cy[a] = cy[a] + v * dy[b]; cz[a] = cz[a] + d * ny[b];
+                            const V3 e0 = u0 - u1, e2 = u2 - u1;
+                            v[b] = u1 + e0 * nz[0] + e2 * nz[1];
+                            d[b] = e0 * dz[0] + e2 * dz[1];
                         }
+                        const V3 e0 = v[0] - v[1], e2 = v[2] - v[1];
+                        cv[a] = v[1] + e0 * ny[0] + e2 * ny[1];
+                        cy[a] = e0 * dy[0] + e2 * dy[1];
+                        cz[a] = d[1] + (d[0] - d[1]) * ny[0] + (d[2] - d[1]) * ny[1];
                     }
                 }
                 [[maybe_unused]] V3 un[E == 8 ? NE : 1];   // P3: the pair's nodes
@@ -864,10 +880,9 @@ k_vertex_points(const SceneDev* __restrict__ scenes, const VWork* __restrict__ w
                     if (q >= NQ) continue;
                     V3 J0 = mk(0, 0, 0), J1 = J0, J2 = J0;
                     if constexpr (E == 9) {
-#pragma unroll
-                        for (int k = 0; k < 3; ++k) {
-                            J0 = J0 + cv[k] * q2_d(a, k); J1 = J1 + cy[k] * q2_n(a, k); J2 = J2 + cz[k] * q2_n(a, k);
-                        }
+                        J0 = (cv[0] - cv[1]) * q2_d(a, 0) + (cv[2] - cv[1]) * q2_d(a, 2);
+                        J1 = cy[1] + (cy[0] - cy[1]) * q2_n(a, 0) + (cy[2] - cy[1]) * q2_n(a, 2);
+                        J2 = cz[1] + (cz[0] - cz[1]) * q2_n(a, 0) + (cz[2] - cz[1]) * q2_n(a, 2);
                     } else {
                         const float4* row = reinterpret_cast<const float4*>(&s_dN[q * NE * 3]);   // 15 x 16 B
 #pragma unroll
