@@ -199,6 +199,33 @@ __device__ __forceinline__ void kadd(float& s, float& c, float v) {
     s = t;
 }
 
+// Sum of a vertex's terms over its t lanes.  In mixed precision the lanes' compensations travel with
+// their sums, and what each addition rounds off (the two-sum, exact whichever term is larger) joins
+// them: the owners of a vertex nearly cancel, and the lanes a launch gives it must not change what
+// the sum keeps.
+__device__ __forceinline__ void lane_sum(float acc[9], float cmp[3], int t, bool mixed) {
+    for (int off = t >> 1; off > 0; off >>= 1) {
+        if (mixed) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const float o = __shfl_xor_sync(0xffffffffu, acc[k], off), e = __shfl_xor_sync(0xffffffffu, cmp[k], off);
+                const float s = acc[k] + o, b = s - acc[k];
+                cmp[k] = (cmp[k] + e) - ((acc[k] - (s - b)) + (o - b));
+                acc[k] = s;
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], off);
+        }
+#pragma unroll
+        for (int k = 3; k < 9; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], off);
+    }
+    if (mixed) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) acc[k] -= cmp[k];
+    }
+}
+
 // Element types whose mixed-precision force is compensated once per owner element, after a
 // plain sum over its quadrature points, instead of once per point: the many-point elements
 // (P3 11 points, Q2 27), where the per-point compensation is a long dependent chain (sweep
@@ -1058,14 +1085,7 @@ __global__ void __launch_bounds__(kBlock, LaneMinBlocks<E>::value) k_vertex(cons
         } else {
             for (; o < oe; o += t) owner_terms<E, MAT>(S, __ldg(S.owners + o), s_dN, mixed, acc, cmp);
         }
-        if (mixed) {
-#pragma unroll
-            for (int k = 0; k < 3; ++k) acc[k] -= cmp[k];
-        }
-        for (int off = t >> 1; off > 0; off >>= 1) {
-#pragma unroll
-            for (int k = 0; k < 9; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], off);
-        }
+        lane_sum(acc, cmp, t, mixed);
         if (active && glane == 0) vertex_epilogue(S, vid, acc, mode, P, red);
         w += gridDim.x;
         if (w >= n_work) break;
@@ -1349,14 +1369,7 @@ k_vbd_substep(const SceneDev* __restrict__ scene, const VWork* __restrict__ work
                     }
                     entry_terms<E, MAT, true>(S, reinterpret_cast<const float*>(cur), s_dN, mixed, acc, cmp);
                 }
-                if (mixed) {
-#pragma unroll
-                    for (int k = 0; k < 3; ++k) acc[k] -= cmp[k];
-                }
-                for (int off = t >> 1; off > 0; off >>= 1) {
-#pragma unroll
-                    for (int k = 0; k < 9; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], off);
-                }
+                lane_sum(acc, cmp, t, mixed);
                 if (active && glane == 0) vertex_epilogue(S, vid, acc, 0, P, nullptr);
             }
             const bool last = c + 1 == n_colours;
