@@ -106,13 +106,14 @@ typedef struct oct_scene_desc {
     int32_t precision;              /* OCT_PREC_* */
     int32_t box_limit;              /* 1: clamp free nodes to [box_min, box_max] each iteration */
     float box_min[3], box_max[3];
-    int32_t threads_per_vertex;     /* 0 = measured default per element, -1 = (vertex, owner)
-                                       pairs packed into warps (one lane per pair; several for
-                                       Q2 and small P3 colours), 1..32 = lanes per vertex (power
-                                       of two; a colour whose vertices average more than 8 owners
-                                       per lane gets wider groups, and the element's measured
-                                       default is widened further where a launch has too few
-                                       vertices to fill the GPU) */
+    int32_t threads_per_vertex;     /* -1 = (vertex, owner) pairs packed into warps (one lane per
+                                       pair; several for Q2), 1..32 = lanes per vertex (power of
+                                       two; a colour whose vertices average more than 8 owners per
+                                       lane gets wider groups): the scene's last bits are then its
+                                       own, alone and in any batch.  0 = measured default per
+                                       element, of which a launch with too few vertices to fill the
+                                       GPU makes wider groups (P3: several lanes per pair), so the
+                                       last bits can depend on what else the launch holds */
     int32_t xpbd_version;           /* OCT_XPBD_* (default OCT_XPBD_OPTISHARED) */
     float mg_linear;                /* multigrid VBD for P2 / Q2 (MG_VBD_FEM,
                                        octopus/include/Dynamic/VBD/MG_VertexBlockDescent.h:52-74):

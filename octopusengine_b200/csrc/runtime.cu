@@ -229,6 +229,7 @@ struct oct_scene {
     float young = 0.f, poisson = 0.f, density = 0.f;   // as described (run metadata)
     int last_substeps = 0;
     bool in_place = true, box = false, has_v0 = false;
+    bool pinned = false;            // the description names the lane mapping: no launch changes it
     bool xpbd_raw = true, xpbd_project = true;   // XPBD update form; false: no projection (OptiGroup)
     // frame graph (oct_scene_set_capture): the sub-steps of one frame, replayed while the
     // frame's (dt, substeps) stay the same
@@ -296,7 +297,7 @@ struct oct_batch {
     int solver = OCT_SOLVER_VBD;    // VBD or XPBD: a batch holds scenes of one solver
     XWork* d_xwork = nullptr;       // XPBD: block items, per group and colour
     struct Group {
-        int element, material, tpv;     // XPBD: tpv holds the raw (V1/V2) update flag
+        int element, material, tpv;     // tpv: mapping_of its scenes; XPBD: the raw (V1/V2) update flag
         bool in_place;
         std::vector<int> off;   // per colour, into the group's part of d_vwork (XPBD: d_xwork)
         std::vector<int> form;  // per colour: launch_form (VBD)
@@ -350,7 +351,9 @@ constexpr int kOwnersPerLane = 8;
 // measured_tpv, used when the description leaves the lanes at 0
 int measured_tpv(int element);
 
-// Lanes of one scene's colour.  least: as above.  width: with the default mapping, lanes for the
+// Lanes of one scene's colour.  least: as above.  width: with the default mapping, unless the
+// description names it (then the lanes, and with them the last bits of a result, are the scene's own
+// whatever else its launches hold), lanes for the
 // owners of the colour's vertex of most owners, one each (P1: three, whose one point is a small
 // part of what a vertex costs: an 81-node sub-step in one block 146 us with 8 lanes, 260 us with
 // 32); else least.
@@ -358,14 +361,14 @@ struct ColourLanes {
     int least = 1, width = 1;
     int at(int div) const { return std::max(least, width / div); }
 };
-ColourLanes colour_lanes(int element, int tpv, int begin, int end, const std::vector<int32_t>& own_off) {
+ColourLanes colour_lanes(int element, int tpv, bool pinned, int begin, int end, const std::vector<int32_t>& own_off) {
     ColourLanes l;
     l.least = l.width = tpv;
     if (tpv <= 0 || end <= begin) return l;
     const int64_t n = end - begin, pairs = (int64_t)own_off[end] - own_off[begin];
     while (l.least < 32 && pairs > (int64_t)kOwnersPerLane * l.least * n) l.least <<= 1;
     l.width = l.least;
-    if (tpv != measured_tpv(element)) return l;
+    if (pinned || tpv != measured_tpv(element)) return l;
     const int each = element == kTetra ? 3 : 1;   // the vertices are in the order of decreasing owner count
     while (l.width < 32 && each * l.width < own_off[begin + 1] - own_off[begin]) l.width <<= 1;
     return l;
@@ -390,12 +393,14 @@ int lane_div(int64_t full) {
 // How a colour launch of `pairs` (vertex, owner) pairs is run: tpv > 0 lane groups; else the
 // packed mapping, 0 one lane per pair, -1 point lanes (k_vertex_points).  Q2 always takes point
 // lanes; P3 while its items are about one wave (frame of 20 sweeps, point lanes / one lane per
-// pair: 1,000 nodes 2.7 / 3.3 ms, 50,653 nodes 3.4 / 4.0, 493,039 nodes 23 / 13).
-int launch_form(int element, int tpv, int64_t pairs) {
-    if (tpv > 0) return tpv;
+// pair: 1,000 nodes 2.7 / 3.3 ms, 50,653 nodes 3.4 / 4.0, 493,039 nodes 23 / 13) and the scenes'
+// descriptions do not name the mapping (mapping -1 instead of 0).
+int launch_form(int element, int mapping, int64_t pairs) {
+    if (mapping > 0) return mapping;
     constexpr int64_t kWavePairs = 12000;
-    return element == kHexa27 || (element == kTetra20 && pairs <= kWavePairs) ? -1 : 0;
+    return element == kHexa27 || (element == kTetra20 && mapping == 0 && pairs <= kWavePairs) ? -1 : 0;
 }
+int mapping_of(const oct_scene* s) { return s->tpv > 0 ? s->tpv : s->pinned ? -1 : 0; }
 
 // Split [begin, end) slots into work items for one scene: block-sized items of 128 / t slots
 // (l, div as above), or packed items of whole vertices up to the kernel's (vertex, owner) pairs
@@ -554,8 +559,8 @@ oct_status build_vertex_work(oct_scene* s) {
     s->max_items = 0;
     for (int k = 0; k + 1 < (int)s->color_off.size(); ++k) {
         const int begin = s->color_off[k], end = s->color_off[k + 1];
-        const ColourLanes l = colour_lanes(s->element, s->tpv, begin, end, s->own_off);
-        s->form.push_back(launch_form(s->element, s->tpv, (int64_t)s->own_off[end] - s->own_off[begin]));
+        const ColourLanes l = colour_lanes(s->element, s->tpv, s->pinned, begin, end, s->own_off);
+        s->form.push_back(launch_form(s->element, mapping_of(s), (int64_t)s->own_off[end] - s->own_off[begin]));
         append_vwork(vw, 0, s->element, begin, end, s->form[k], l, lane_div((int64_t)l.width * (end - begin)), s->own_off);
         s->vwork_off.push_back((int)vw.size());
         s->max_items = std::max(s->max_items, s->vwork_off[k + 1] - s->vwork_off[k]);
@@ -685,6 +690,7 @@ oct_status build_scene(oct_ctx* c, const oct_scene_desc* d, oct_scene* s) {
     s->box = d->box_limit != 0;
     s->has_v0 = d->initial_velocity != nullptr;
     s->tpv = d->threads_per_vertex < 0 ? 0 : d->threads_per_vertex;
+    s->pinned = d->threads_per_vertex != 0;
     if (d->threads_per_vertex < -1 || (s->tpv != 0 && s->tpv != 1 && s->tpv != 2 && s->tpv != 4 && s->tpv != 8 &&
                                        s->tpv != 16 && s->tpv != 32))
         return fail(c, OCT_EINVAL, "threads_per_vertex must be -1 (packed), 0 (default) or a power of two <= 32");
@@ -1923,12 +1929,12 @@ oct_status oct_batch_create(oct_ctx* c, oct_scene* const* scenes, int n, oct_bat
                 append_xwork(cw[k], i, s->elem_off[k], s->elem_off[k + 1], xpbd_elements_per_block(s->element));
             continue;
         }
-        auto key = std::make_pair(std::make_pair(s->element, s->material), std::make_pair(s->tpv, s->in_place ? 1 : 0));
+        auto key = std::make_pair(std::make_pair(s->element, s->material), std::make_pair(mapping_of(s), s->in_place ? 1 : 0));
         auto it = gid.find(key);
         if (it == gid.end()) {
             it = gid.emplace(key, (int)b->groups.size()).first;
             oct_batch::Group g;
-            g.element = s->element; g.material = s->material; g.tpv = s->tpv; g.in_place = s->in_place;
+            g.element = s->element; g.material = s->material; g.tpv = mapping_of(s); g.in_place = s->in_place;
             b->groups.push_back(g);
             gwork.emplace_back();
             members.emplace_back();
@@ -1944,7 +1950,8 @@ oct_status oct_batch_create(oct_ctx* c, oct_scene* const* scenes, int n, oct_bat
             for (int i : members[g]) {
                 const oct_scene* s = scenes[i];
                 const bool has = k < s->n_colors;
-                l.push_back(has ? colour_lanes(s->element, s->tpv, s->color_off[k], s->color_off[k + 1], s->own_off) : ColourLanes());
+                l.push_back(has ? colour_lanes(s->element, s->tpv, s->pinned, s->color_off[k], s->color_off[k + 1], s->own_off)
+                                : ColourLanes());
                 if (!has) continue;
                 full += (int64_t)l.back().width * (s->color_off[k + 1] - s->color_off[k]);
                 pairs += s->own_off[s->color_off[k + 1]] - s->own_off[s->color_off[k]];
@@ -2149,7 +2156,7 @@ oct_status oct_batch_group_info(oct_batch* b, int g, int32_t* element, int32_t* 
     int64_t nv = 0;
     const double tf = vbd_term_flops(G.element, G.material);
     for (auto* s : b->scenes) {
-        if (s->element != G.element || s->material != G.material || s->tpv != G.tpv || s->in_place != G.in_place) continue;
+        if (s->element != G.element || s->material != G.material || mapping_of(s) != G.tpv || s->in_place != G.in_place) continue;
         const int64_t free_nodes = s->n_nodes - s->n_fixed;
         const int64_t terms = (int64_t)s->n_elements * s->ne * s->nq;   // sum over vertices of owners x Q
         fl += tf * (double)terms * (double)free_nodes / (double)s->n_nodes;
@@ -2205,6 +2212,7 @@ oct_status oct_scene_set_mapping(oct_scene* s, int tpv) {
     }
     OCT_CUDA(s->ctx, cudaStreamSynchronize(s->ctx->stream));
     s->tpv = t;
+    s->pinned = false;
     drop_frame_graph(s);
     return build_vertex_work(s);
 }
@@ -2251,7 +2259,10 @@ oct_status oct_autotune_mapping(oct_ctx* c, oct_scene* const* scenes, int n, flo
         for (auto* s : list) { max_val = std::max(max_val, s->max_valence); entries = entries && s->h.ent; }
         std::vector<int> cands = {1, 2, 4, 8, 16, 32};
         if (max_val <= 32 && entries) cands.insert(cands.begin(), -1);
-        const std::vector<int> old = [&] { std::vector<int> v; for (auto* s : list) v.push_back(s->tpv); return v; }();
+        // the candidates are timed as oct_scene_set_mapping sets them; host fields only
+        std::vector<std::pair<int, bool>> old;
+        for (auto* s : list) { old.push_back({s->tpv, s->pinned}); s->pinned = false; }
+        auto put_back = [&] { for (size_t i = 0; i < list.size(); ++i) { list[i]->tpv = old[i].first; list[i]->pinned = old[i].second; } };
         // the measured default is timed first and kept unless a candidate is clearly faster:
         // candidates that differ little (the per-colour lane rule makes neighbours build
         // nearly the same items) must not switch on timing noise
@@ -2262,11 +2273,11 @@ oct_status oct_autotune_mapping(oct_ctx* c, oct_scene* const* scenes, int n, flo
         float best_ms = 1e30f, dflt_ms = 1e30f;
         int best = dflt;
         for (int cand : cands) {
-            for (auto* s : list) s->tpv = cand < 0 ? 0 : cand;   // host field only: the batch builds its own tables
+            for (auto* s : list) s->tpv = cand < 0 ? 0 : cand;   // the batch builds its own tables
             oct_batch* b = nullptr;
             oct_status st = oct_batch_create(c, list.data(), (int)list.size(), &b);
             if (st) {
-                for (size_t i = 0; i < list.size(); ++i) list[i]->tpv = old[i];
+                put_back();
                 return st;
             }
             float ms = 1e30f, t = 0.f;
@@ -2277,13 +2288,13 @@ oct_status oct_autotune_mapping(oct_ctx* c, oct_scene* const* scenes, int n, flo
             }
             oct_batch_destroy(b);
             if (st) {
-                for (size_t i = 0; i < list.size(); ++i) list[i]->tpv = old[i];
+                put_back();
                 return st;
             }
             if (cand == dflt) dflt_ms = ms;
             if (ms < best_ms && (cand == dflt || ms < 0.97f * dflt_ms)) { best_ms = ms; best = cand; }
         }
-        for (size_t i = 0; i < list.size(); ++i) list[i]->tpv = old[i];
+        put_back();
         for (auto* s : list) {
             oct_status st = oct_scene_set_mapping(s, best);
             if (st) return st;
