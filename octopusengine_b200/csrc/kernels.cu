@@ -1245,10 +1245,13 @@ __global__ void k_constraints(const SceneDev* __restrict__ scenes, const NWork* 
 // owner entry in flight while it waits for the others.  The colours' work items, lanes and
 // arithmetic are those of k_vertex, so the results are the same bits.
 //
-// Blocks of 512 threads, at most one per SM, are four sub-blocks of 128, each taking items of the
-// colour in turn (first one per SM).  A scene whose colours fit a few items runs in one block, and
-// its barrier is __syncthreads.  The SceneDev is copied to shared memory: the barrier's acquire
-// empties L1.
+// Blocks, at most one per SM, are sub-blocks of 128 threads, each taking items of the colour in turn
+// (first one per SM).  There are no more of them than the largest colour has items for, one or two
+// in a grid of several blocks: the launch holds its part of the SMs while it waits in barriers, and
+// with four everywhere (the whole register file) the sub-steps of two contexts took turns (frames of
+// two contexts at once, four sub-blocks / one: 18,785-node P1 655 / 414 us, Q1 1,857 / 1,118; alone
+// the same).  A scene whose colours fit a few items runs in one block, of up to four, and its
+// barrier is __syncthreads.  The SceneDev is copied to shared memory: the barrier's acquire empties L1.
 constexpr int kSubBlocks = 4;
 
 // Barrier over the grid: bar[0] counts arrivals, bar[1] blocks that have left.  The wait has an
@@ -1313,7 +1316,7 @@ k_vbd_substep(const SceneDev* __restrict__ scene, const VWork* __restrict__ work
     const SceneDev& S = s_scene;
     const unsigned long long stream = policy_stream();
     const int lane = threadIdx.x & 31, tid = threadIdx.x & (kBlock - 1);
-    const int first = (threadIdx.x / kBlock) * gridDim.x + blockIdx.x, step = gridDim.x * kSubBlocks;
+    const int first = (threadIdx.x / kBlock) * gridDim.x + blockIdx.x, step = gridDim.x * (blockDim.x / kBlock);
     const int node0 = blockIdx.x * blockDim.x + threadIdx.x, nodes = gridDim.x * blockDim.x;
     const bool mixed = S.precision != 0, cheb = rho > 0.f;
     int t = 1, glane = 0, o = 0, oe = 0, vid = -1;   // this lane's part of its next item
@@ -2629,14 +2632,14 @@ void launch_vertex(int element, int material, const SceneDev* scenes, const VWor
 namespace {
 template <int E>
 bool substep_mat(int mat, const SceneDev* scene, const VWork* work, const int* colour_off, int n_colours, int iterations,
-                 float rho, unsigned* bar, int grid, const StepParams& P, cudaStream_t st) {
+                 float rho, unsigned* bar, int grid, int subs, const StepParams& P, cudaStream_t st) {
     auto go = [&](auto kernel) {
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeCooperative;
         at[0].val.cooperative = 1;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(grid);
-        cfg.blockDim = dim3(kSubBlocks * kBlock);
+        cfg.blockDim = dim3(subs * kBlock);
         cfg.stream = st;
         cfg.attrs = at;
         cfg.numAttrs = grid > 1 ? 1 : 0;
@@ -2652,11 +2655,12 @@ bool substep_mat(int mat, const SceneDev* scene, const VWork* work, const int* c
 }  // namespace
 
 bool launch_vbd_substep(int element, int material, const SceneDev* scene, const VWork* work, const int* colour_off,
-                        int n_colours, int iterations, float rho, unsigned* bar, int grid, const StepParams& P, cudaStream_t st) {
+                        int n_colours, int iterations, float rho, unsigned* bar, int grid, int subs, const StepParams& P,
+                        cudaStream_t st) {
     switch (element) {
-        case 3: return substep_mat<3>(material, scene, work, colour_off, n_colours, iterations, rho, bar, grid, P, st);
-        case 6: return substep_mat<6>(material, scene, work, colour_off, n_colours, iterations, rho, bar, grid, P, st);
-        case 7: return substep_mat<7>(material, scene, work, colour_off, n_colours, iterations, rho, bar, grid, P, st);
+        case 3: return substep_mat<3>(material, scene, work, colour_off, n_colours, iterations, rho, bar, grid, subs, P, st);
+        case 6: return substep_mat<6>(material, scene, work, colour_off, n_colours, iterations, rho, bar, grid, subs, P, st);
+        case 7: return substep_mat<7>(material, scene, work, colour_off, n_colours, iterations, rho, bar, grid, subs, P, st);
         default: return false;
     }
 }

@@ -15,12 +15,13 @@ void prepare_vertex(int element, int material);
 // mode 0: VBD solve, 1: VBD residual (red[0] += |r|, red[1] = max |r|)
 void launch_vertex(int element, int material, const SceneDev* scenes, const VWork* work, int n_work, int form, int mode,
                    const StepParams& P, double* red, cudaStream_t st);
-// One VBD sub-step of one scene in one cooperative launch of `grid` blocks (at most one per SM);
+// One VBD sub-step of one scene in one cooperative launch of `grid` blocks (at most one per SM) of
+// `subs` (1 to 4) groups of 128 threads;
 // work: the scene's lane-group items, colour_off: n_colours + 1 offsets into it (device), bar: two
 // zeroed words.  rho 0: no Chebyshev.
 bool launch_vbd_substep(int element, int material, const SceneDev* scene, const VWork* work, const int* colour_off,
-                        int n_colours, int iterations, float rho, unsigned* bar, int grid, const StepParams& P,
-                        cudaStream_t st);
+                        int n_colours, int iterations, float rho, unsigned* bar, int grid, int subs,
+                        const StepParams& P, cudaStream_t st);
 void launch_commit(const SceneDev* scenes, const VWork* work, int n_work, cudaStream_t st);
 // Explicit sub-step: the element-centric force pass (one force per (element, local node), written
 // to the owner's place in contrib, n_elements x NE float4; damped: the scene has damping), then per

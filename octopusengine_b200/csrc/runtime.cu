@@ -28,7 +28,7 @@ using namespace octb;
 
 namespace {
 constexpr int kBlockThreads = 128;
-constexpr int kSubBlocks = 4;   // k_vbd_substep: groups of kBlockThreads per block
+constexpr int kSubBlocks = 4;   // k_vbd_substep: groups of kBlockThreads per block, at most
 
 // NVTX ranges around frames, sub-steps and colour sweeps (host side; a profiler shows them on
 // the timeline, and without one they cost a pointer test).
@@ -1136,10 +1136,13 @@ void vbd_substep(oct_scene* s, float dt) {
     };
     if (one_launch(s)) {
         const int sms = sm_count(c);
+        // no more groups per block than the largest colour has items for: the launch stays on the
+        // SMs for the whole sub-step, and what it does not hold of them other streams can use
         const int grid = s->max_items <= 2 * kSubBlocks ? 1 : std::min(s->max_items, sms);
+        const int subs = std::min((s->max_items + grid - 1) / grid, kSubBlocks);
         const bool taken = c->refuse > 0 ? (--c->refuse, false) :
             launch_vbd_substep(s->element, s->material, s->d_scene, s->d_vwork, s->d_vwork_off, s->n_colors, s->iterations,
-                               cheb ? s->rho : 0.f, s->d_bar, grid, P, st);
+                               cheb ? s->rho : 0.f, s->d_bar, grid, subs, P, st);
         if (taken) {
             c->launches++;
             consumed();
