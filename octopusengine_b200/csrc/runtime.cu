@@ -1457,7 +1457,9 @@ oct_status oct_scene_sync(oct_scene* s) {
     if (!s) return OCT_EINVAL;
     oct_ctx* c = s->ctx;
     const oct_status st = sync_and_check(c);
-    cudaEventElapsedTime(&c->last_ms, c->ev0, c->ev1);
+    // before a context's first step its events are not recorded: no time, and no error left behind
+    // for the next step to report
+    if (cudaEventElapsedTime(&c->last_ms, c->ev0, c->ev1) != cudaSuccess) cudaGetLastError();
     return st;
 }
 

@@ -53,3 +53,14 @@ def test_a_refused_launch_falls_back_to_launches_per_colour(ctx, element, cells,
     np.testing.assert_array_equal(s.get_position(), twin.get_position())
     np.testing.assert_array_equal(s.get_velocity(), twin.get_velocity())
     assert np.abs(s.get_velocity()).max() > 0
+
+
+def test_a_sync_before_the_first_step_leaves_no_error(built):
+    import octopusengine_b200 as ob
+    c = ob.Context(0, 1 << 28)
+    X, T = O.beam_mesh(O.TETRA, (2, 1, 1), (1.0, 0.5, 0.5))
+    s = ob.Scene(c, O.TETRA, X, T, iterations=2)
+    s.sync()
+    s.step(1 / 60, 1)
+    assert s.status() == 0
+    c.close()
