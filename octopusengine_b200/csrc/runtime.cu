@@ -38,84 +38,12 @@ struct Range {
 };
 constexpr int kNodeChunk = 256;
 
-// Pinned staging of one transfer between a context and pageable host memory: a ring of chunks with
-// an event each, and room for the error word and reductions.
-constexpr size_t kIoChunk = 256 << 10;
-constexpr int kIoSlots = 8;
-struct IoBuffer {
-    int device = 0;
-    char* ring = nullptr;        // kIoSlots chunks
-    double* small = nullptr;     // 8 doubles behind the ring
-    cudaEvent_t ev[kIoSlots] = {};
-};
-
-// Staging buffers are lent for the length of a transfer, so a process has as many as it has
-// transfers under way at once (2 MB each; pinning one takes milliseconds, which is why they are
-// not a context's own).  The first context of a device brings one; at most kKept are kept between
-// transfers, and all are given back with the last context.
-struct IoPool {
-    static constexpr size_t kKept = 4;
-    std::mutex mu;
-    std::vector<IoBuffer*> idle;
-    int contexts = 0;
-    static void destroy(IoBuffer* b) {
-        for (auto e : b->ev) if (e) cudaEventDestroy(e);
-        if (b->ring) cudaFreeHost(b->ring);
-        delete b;
-    }
-    IoBuffer* take(int device) {   // null when none can be had
-        {
-            std::lock_guard<std::mutex> lock(mu);
-            for (size_t i = 0; i < idle.size(); ++i)
-                if (idle[i]->device == device) {
-                    IoBuffer* b = idle[i];
-                    idle.erase(idle.begin() + i);
-                    return b;
-                }
-        }
-        auto* b = new IoBuffer();
-        b->device = device;
-        bool ok = cudaHostAlloc((void**)&b->ring, kIoChunk * kIoSlots + 64, cudaHostAllocPortable) == cudaSuccess;
-        for (auto& e : b->ev) ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
-        if (!ok) {
-            cudaGetLastError();
-            destroy(b);
-            return nullptr;
-        }
-        b->small = reinterpret_cast<double*>(b->ring + kIoChunk * kIoSlots);
-        return b;
-    }
-    void give(IoBuffer* b) {
-        if (!b) return;
-        std::unique_lock<std::mutex> lock(mu);
-        if (contexts > 0 && idle.size() < kKept) { idle.push_back(b); return; }
-        lock.unlock();
-        destroy(b);
-    }
-    void enter(int device) {
-        { std::lock_guard<std::mutex> lock(mu); ++contexts; }
-        give(take(device));
-    }
-    void leave() {
-        std::vector<IoBuffer*> gone;
-        {
-            std::lock_guard<std::mutex> lock(mu);
-            if (--contexts == 0) gone.swap(idle);
-        }
-        for (auto* b : gone) destroy(b);
-    }
-};
-IoPool& io_pool() {
-    static IoPool* pool = new IoPool();   // outlives every context, those of static objects too
-    return *pool;
-}
-struct IoLoan {
-    IoBuffer* b;
-    explicit IoLoan(int device) : b(io_pool().take(device)) {}
-    ~IoLoan() { io_pool().give(b); }
-    IoLoan(const IoLoan&) = delete;
-    IoLoan& operator=(const IoLoan&) = delete;
-};
+// A context's pinned block, for the error word, reductions and node states that fit it, and the
+// number of uses after which it is made: pinning and unpinning cost 1.3 ms whatever the size, a use
+// saves 4.5 us (frame of 81 nodes with both getters 218 -> 205 us), and a context that lives for a few
+// frames never pins.
+constexpr size_t kIoBytes = 256 << 10;
+constexpr int kIoAfter = 32;
 }  // namespace
 
 struct oct_ctx {
@@ -129,6 +57,9 @@ struct oct_ctx {
     uint64_t launches = 0;
     bool tables[10] = {false};
     int sms = 0;         // streaming multiprocessors (sm_count)
+    std::mutex io_mu;          // guards the pinned block (IoLoan)
+    char* io = nullptr;
+    int io_uses = 0;
     int refuse = 0;      // oct_ctx_refuse_probe: cooperative launches still to be taken as refused
     std::mutex mu;       // guards the budget accounting and the shape-table upload
     std::mutex err_mu;   // guards err (scenes may be created from several host threads)
@@ -473,15 +404,40 @@ oct_status error_status(oct_ctx* c, int e) {
     return OCT_OK;
 }
 
+// The context's pinned block for the length of one transfer.  p is null while the context has none,
+// or another thread has it: the transfer then goes to the caller's memory itself.
+struct IoLoan {
+    oct_ctx* c;
+    char* p = nullptr;
+    explicit IoLoan(oct_ctx* ctx) : c(ctx) {
+        if (!c->io_mu.try_lock()) return;
+        if (!c->io && c->io_uses <= kIoAfter && ++c->io_uses > kIoAfter) {   // tried once
+            int current = 0;
+            cudaGetDevice(&current);
+            cudaSetDevice(c->device);
+            if (cudaHostAlloc((void**)&c->io, kIoBytes, cudaHostAllocPortable) != cudaSuccess) {
+                cudaGetLastError();
+                c->io = nullptr;
+            }
+            cudaSetDevice(current);
+        }
+        p = c->io;
+        if (!p) c->io_mu.unlock();
+    }
+    ~IoLoan() { if (p) c->io_mu.unlock(); }
+    IoLoan(const IoLoan&) = delete;
+    IoLoan& operator=(const IoLoan&) = delete;
+};
+
 // Waits for the context's stream, with `n` (at most 7) doubles of device reductions into out, and
 // reports the error word.  One wait: the word and the values come back behind the work.
 oct_status sync_and_check(oct_ctx* c, const double* red = nullptr, double* out = nullptr, int n = 0) {
-    IoLoan io(c->device);
+    IoLoan io(c);
     double local[8];
-    double* h = io.b ? io.b->small : local;
-    if (red) OCT_CUDA(c, cudaMemcpyAsync(h + 1, red, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    const cudaError_t e = cudaMemcpyAsync(h, c->d_error, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
-    const cudaError_t es = cudaStreamSynchronize(c->stream);   // before the buffer goes back, whatever failed
+    double* h = io.p ? reinterpret_cast<double*>(io.p) : local;
+    cudaError_t e = red ? cudaMemcpyAsync(h + 1, red, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream) : cudaSuccess;
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h, c->d_error, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
+    const cudaError_t es = cudaStreamSynchronize(c->stream);   // nothing may land in h after this
     OCT_CUDA(c, e);
     OCT_CUDA(c, es);
     std::copy(h + 1, h + 1 + n, out);
@@ -490,64 +446,19 @@ oct_status sync_and_check(oct_ctx* c, const double* red = nullptr, double* out =
     return error_status(c, word);
 }
 
-// Ordinary host memory, unknown to CUDA: only that is staged.
+// Ordinary host memory, unknown to CUDA.
 bool pageable(const void* p) {
     cudaPointerAttributes a;
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return false; }
     return a.type == cudaMemoryTypeUnregistered;
 }
 
-// Device to host on the context's stream; returns when `out` holds the values.  A copy into
-// pageable memory goes through the driver's own staging at 5 GB/s (1.7 MB in 330 us); here chunks
-// arrive in the pinned ring and are copied out while the next ones are in flight (190 us, most
-// of it the first touch of the caller's pages).  Pinned memory is the copy's target itself.
+// Device to host on the context's stream; returns when `out` holds the values.  Large copies into
+// pageable memory are left to the driver's staging: a pinned ring of the context's own, copied out
+// chunk by chunk, was no faster (set and read back 140,481 nodes' quantities 304 us, 335 with it).
 oct_status copy_out(oct_ctx* c, void* out, const void* d, size_t bytes) {
-    IoLoan io(c->device);
-    if (!io.b || !pageable(out)) {
-        OCT_CUDA(c, cudaMemcpyAsync(out, d, bytes, cudaMemcpyDeviceToHost, c->stream));
-        OCT_CUDA(c, cudaStreamSynchronize(c->stream));
-        return OCT_OK;
-    }
-    const size_t n = (bytes + kIoChunk - 1) / kIoChunk;
-    auto length = [&](size_t i) { return std::min(kIoChunk, bytes - i * kIoChunk); };
-    cudaError_t e = cudaSuccess;
-    auto issue = [&](size_t i) {
-        const size_t k = i % kIoSlots;
-        if (e == cudaSuccess) e = cudaMemcpyAsync(io.b->ring + k * kIoChunk, (const char*)d + i * kIoChunk, length(i), cudaMemcpyDeviceToHost, c->stream);
-        if (e == cudaSuccess) e = cudaEventRecord(io.b->ev[k], c->stream);
-    };
-    for (size_t i = 0; i < n && i < kIoSlots; ++i) issue(i);
-    for (size_t i = 0; i < n && e == cudaSuccess; ++i) {
-        const size_t k = i % kIoSlots;
-        if ((e = cudaEventSynchronize(io.b->ev[k])) != cudaSuccess) break;
-        std::memcpy((char*)out + i * kIoChunk, io.b->ring + k * kIoChunk, length(i));
-        if (i + kIoSlots < n) issue(i + kIoSlots);
-    }
-    if (e != cudaSuccess) cudaStreamSynchronize(c->stream);   // nothing may land in the ring after this
-    OCT_CUDA(c, e);
-    return OCT_OK;
-}
-
-// Host to device on the context's stream, then `after` (work that reads it); returns when the
-// stream has drained, so the caller may reuse `in`.
-template <class F> oct_status copy_in(oct_ctx* c, void* d, const void* in, size_t bytes, F after) {
-    IoLoan io(c->device);
-    cudaError_t e = cudaSuccess;
-    if (!io.b || !pageable(in)) {
-        e = cudaMemcpyAsync(d, in, bytes, cudaMemcpyHostToDevice, c->stream);
-    } else {
-        for (size_t i = 0; i * kIoChunk < bytes && e == cudaSuccess; ++i) {
-            const size_t k = i % kIoSlots, len = std::min(kIoChunk, bytes - i * kIoChunk);
-            if (i >= kIoSlots) e = cudaEventSynchronize(io.b->ev[k]);
-            std::memcpy(io.b->ring + k * kIoChunk, (const char*)in + i * kIoChunk, len);
-            if (e == cudaSuccess) e = cudaMemcpyAsync((char*)d + i * kIoChunk, io.b->ring + k * kIoChunk, len, cudaMemcpyHostToDevice, c->stream);
-            if (e == cudaSuccess) e = cudaEventRecord(io.b->ev[k], c->stream);
-        }
-    }
-    if (e == cudaSuccess) after();
-    const cudaError_t es = cudaStreamSynchronize(c->stream);
-    OCT_CUDA(c, e);
-    OCT_CUDA(c, es);
+    OCT_CUDA(c, cudaMemcpyAsync(out, d, bytes, cudaMemcpyDeviceToHost, c->stream));
+    OCT_CUDA(c, cudaStreamSynchronize(c->stream));
     return OCT_OK;
 }
 
@@ -1246,18 +1157,18 @@ void explicit_substep(oct_scene* s, float dt) {
 }
 
 // Node state out as n x 3 floats (the caller's buffer may be pinned or pageable); returns when
-// `out` holds the values.  A state of one chunk is written by the kernel into the pinned ring
-// itself, a larger one goes through the device buffer and copy_out.
+// `out` holds the values.  A state that fits the context's pinned block is written there by the
+// kernel itself; else it goes through the device buffer.
 oct_status read_nodes(oct_scene* s, const float4* d, float* out, bool add_rest) {
     oct_ctx* c = s->ctx;
     oct_status st;
     const size_t bytes = sizeof(float) * 3 * s->n_nodes;
-    if (bytes <= kIoChunk && pageable(out)) {
-        IoLoan io(c->device);
-        if (io.b) {
-            launch_nodes_out(d, add_rest ? s->h.X : nullptr, (float*)io.b->ring, s->n_nodes, c->stream);
+    if (bytes <= kIoBytes && pageable(out)) {
+        IoLoan io(c);
+        if (io.p) {
+            launch_nodes_out(d, add_rest ? s->h.X : nullptr, (float*)io.p, s->n_nodes, c->stream);
             OCT_CUDA(c, cudaStreamSynchronize(c->stream));
-            std::memcpy(out, io.b->ring, bytes);
+            std::memcpy(out, io.p, bytes);
             return OCT_OK;
         }
     }
@@ -1272,8 +1183,10 @@ oct_status write_nodes(oct_scene* s, const float* in, float4* d, bool sub_rest) 
     oct_ctx* c = s->ctx;
     oct_status st;
     if (!s->d_io && (st = s->mem.alloc(s->d_io, (size_t)s->n_nodes * 3))) return st;
-    return copy_in(c, s->d_io, in, sizeof(float) * 3 * s->n_nodes,
-                   [&] { launch_nodes_in(s->d_io, sub_rest ? s->h.X : nullptr, d, s->n_nodes, c->stream); });
+    OCT_CUDA(c, cudaMemcpyAsync(s->d_io, in, sizeof(float) * 3 * s->n_nodes, cudaMemcpyHostToDevice, c->stream));
+    launch_nodes_in(s->d_io, sub_rest ? s->h.X : nullptr, d, s->n_nodes, c->stream);
+    OCT_CUDA(c, cudaStreamSynchronize(c->stream));
+    return OCT_OK;
 }
 
 void run_frame(oct_scene* s, float sub, int substeps) {
@@ -1332,7 +1245,6 @@ oct_status oct_ctx_create(int device, size_t budget, oct_ctx** out) {
         delete c;
         return OCT_ECUDA;
     }
-    io_pool().enter(device);
     *out = c;
     return OCT_OK;
 }
@@ -1345,7 +1257,7 @@ oct_status oct_ctx_destroy(oct_ctx* c) {
         trim_cache(c);
     }
     cudaFree(c->d_error);
-    io_pool().leave();
+    if (c->io) cudaFreeHost(c->io);
     cudaEventDestroy(c->ev0);
     cudaEventDestroy(c->ev1);
     cudaStreamDestroy(c->stream);
