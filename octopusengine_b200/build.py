@@ -19,9 +19,10 @@ BUILD = os.path.join(PKG, "_build")
 LIB = os.path.join(PKG, "liboctb.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-# split-compile: the kernel instantiations of one source are optimised in parallel (kernels.cu
-# takes 75 s on eight cores instead of 230)
-FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-split-compile=8", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
+# kernels.cu takes four minutes.  -split-compile would take 75 s on eight cores, but its code differs
+# from run to run of the compiler: the same source gave 3.45 or 3.90 ms per frame of 50,653 P3 nodes,
+# 684 or 708 us for XPBD P2, and other roundings.
+FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
          "-Xcompiler", "-Wall", "-I", os.path.join(ROOT, "include"), "-I", CSRC]
 EXTRA = os.environ.get("OCTB_NVCC_FLAGS", "").split()
 
