@@ -4,6 +4,7 @@
 // (element type, colour) captured in a CUDA graph.
 #include <algorithm>
 #include <array>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -44,6 +45,16 @@ constexpr int kNodeChunk = 256;
 // frames never pins.
 constexpr size_t kIoBytes = 256 << 10;
 constexpr int kIoAfter = 32;
+
+// Per device, the groups of 128 threads that the one-launch sub-steps of contexts with work in flight
+// hold (oct_ctx::held), and how many an SM may hold: half of what its registers have room for.  A
+// launch that would exceed it takes the launch path, of the same bits, which shares the SMs kernel by
+// kernel: frames of 4 / 8 contexts at once, without a limit and with it, 26,353-node P2 2,436 / 4,897
+// and 2,127 / 3,767 us, 60,625-node P2 3,468 / 7,031 and 2,885 / 5,156, 29,241-node P1 819 / 1,629
+// and 724 / 1,264.  A frame that is captured is not asked, its replays are counted.
+constexpr int kDevices = 64;
+constexpr int kHeldPerSm = 2;
+std::atomic<int> g_held[kDevices];
 }  // namespace
 
 struct oct_ctx {
@@ -60,6 +71,8 @@ struct oct_ctx {
     std::mutex io_mu;          // guards the pinned block (IoLoan)
     char* io = nullptr;
     int io_uses = 0;
+    bool capturing = false;    // a frame graph (oct_scene_step)
+    std::atomic<int> held{0};  // this context's part of g_held, until its stream is waited for
     int refuse = 0;      // oct_ctx_refuse_probe: cooperative launches still to be taken as refused
     std::mutex mu;       // guards the budget accounting and the shape-table upload
     std::mutex err_mu;   // guards err (scenes may be created from several host threads)
@@ -169,6 +182,7 @@ struct oct_scene {
     float frame_dt = -1.f;
     int frame_substeps = 0;
     uint64_t frame_launches = 0;
+    int frame_held = 0;             // groups that its one-launch sub-steps hold
     std::mt19937 rng;
     std::vector<int32_t> colors, vids, color_off;   // colour-sorted slots
     std::vector<int32_t> own_off;                    // owner CSR offsets in slot order (host copy)
@@ -404,6 +418,9 @@ oct_status error_status(oct_ctx* c, int e) {
     return OCT_OK;
 }
 
+// Notes that the context's work in flight holds n groups of the device's SMs (0: none).
+void hold(oct_ctx* c, int n) { g_held[c->device % kDevices] += n - c->held.exchange(n); }
+
 // The context's pinned block for the length of one transfer.  p is null while the context has none,
 // or another thread has it: the transfer then goes to the caller's memory itself.
 struct IoLoan {
@@ -438,6 +455,7 @@ oct_status sync_and_check(oct_ctx* c, const double* red = nullptr, double* out =
     cudaError_t e = red ? cudaMemcpyAsync(h + 1, red, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream) : cudaSuccess;
     if (e == cudaSuccess) e = cudaMemcpyAsync(h, c->d_error, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
     const cudaError_t es = cudaStreamSynchronize(c->stream);   // nothing may land in h after this
+    hold(c, 0);
     OCT_CUDA(c, e);
     OCT_CUDA(c, es);
     std::copy(h + 1, h + 1 + n, out);
@@ -1051,16 +1069,21 @@ void vbd_substep(oct_scene* s, float dt) {
         // SMs for the whole sub-step, and what it does not hold of them other streams can use
         const int grid = s->max_items <= 2 * kSubBlocks ? 1 : std::min(s->max_items, sms);
         const int subs = std::min((s->max_items + grid - 1) / grid, kSubBlocks);
-        const bool taken = c->refuse > 0 ? (--c->refuse, false) :
-            launch_vbd_substep(s->element, s->material, s->d_scene, s->d_vwork, s->d_vwork_off, s->n_colors, s->iterations,
-                               cheb ? s->rho : 0.f, s->d_bar, grid, subs, P, st);
-        if (taken) {
-            c->launches++;
-            consumed();
-            return;
+        const bool room = c->capturing || g_held[c->device % kDevices] - c->held + grid * subs <= kHeldPerSm * sms;
+        if (room) {
+            const bool taken = c->refuse > 0 ? (--c->refuse, false) :
+                launch_vbd_substep(s->element, s->material, s->d_scene, s->d_vwork, s->d_vwork_off, s->n_colors, s->iterations,
+                                   cheb ? s->rho : 0.f, s->d_bar, grid, subs, P, st);
+            if (taken) {
+                if (c->capturing) s->frame_held = grid * subs;
+                else hold(c, grid * subs);
+                c->launches++;
+                consumed();
+                return;
+            }
+            cudaGetLastError();   // fewer co-resident blocks than SMs (a partitioned device): the same work, a launch per colour
+            s->one_launch_refused = true;
         }
-        cudaGetLastError();   // fewer co-resident blocks than SMs (a partitioned device): the same work, a launch per colour
-        s->one_launch_refused = true;
     }
     launch_predict(s->d_scene, s->d_nwork, s->n_nwork, 0, 0, cheb ? 1 : 0, P, st);
     c->launches++;
@@ -1258,6 +1281,7 @@ oct_status oct_ctx_destroy(oct_ctx* c) {
     }
     cudaFree(c->d_error);
     if (c->io) cudaFreeHost(c->io);
+    hold(c, 0);
     cudaEventDestroy(c->ev0);
     cudaEventDestroy(c->ev1);
     cudaStreamDestroy(c->stream);
@@ -1326,7 +1350,10 @@ oct_status oct_scene_step(oct_scene* s, float frame_dt, int substeps) {
         drop_frame_graph(s);
         const uint64_t l0 = c->launches;
         OCT_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+        c->capturing = true;
+        s->frame_held = 0;
         run_frame(s, sub, substeps);
+        c->capturing = false;
         cudaGraph_t g = nullptr;
         const cudaError_t e = cudaStreamEndCapture(c->stream, &g);
         s->frame_launches = c->launches - l0;
@@ -1349,6 +1376,7 @@ oct_status oct_scene_step(oct_scene* s, float frame_dt, int substeps) {
     if (graph) {
         OCT_CUDA(c, cudaGraphLaunch(s->frame_exec, c->stream));
         c->launches += s->frame_launches;
+        if (s->frame_held) hold(c, s->frame_held);
     } else {
         run_frame(s, sub, substeps);
     }

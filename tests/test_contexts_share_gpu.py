@@ -1,6 +1,7 @@
 """Two contexts, each stepped by its own thread, share the GPU: a scene's launches leave room on the
 SMs for another's.  Medium scenes, whose one-launch sub-steps hold as many blocks as there are SMs
-or close to it: if they took turns, two would take twice as long as one."""
+or close to it: if they took turns, two would take twice as long as one.  While another context's
+launches hold the SMs, a scene takes the launch path, to the same bits."""
 import threading
 import time
 
@@ -46,3 +47,26 @@ def test_two_contexts_overlap(built, element, cells):
     for c in ctxs:
         c.close()
     assert two < 1.5 * one, (one, two)
+
+
+def test_a_context_gives_way_to_one_in_flight(built):
+    import octopusengine_b200 as ob
+    X, T = O.beam_mesh(O.TETRA10, (36, 9, 9), (2.25, 0.5625, 0.5625))   # two groups of threads on most SMs
+    ctxs = [ob.Context(0, 1 << 30) for _ in range(2)]
+    a, b = [ob.Scene(c, O.TETRA10, X, T, iterations=4, young=1e6) for c in ctxs]
+
+    def launches(s):
+        n = s.ctx.launch_count()
+        s.step(1 / 60, 3)
+        return s.ctx.launch_count() - n
+
+    assert launches(a) == 3 and launches(b) == 3
+    a.step(1 / 60, 3, sync=False)
+    assert launches(b) > 3
+    a.sync()
+    assert launches(b) == 3
+    a.step(1 / 60, 3)
+    np.testing.assert_array_equal(a.get_position(), b.get_position())
+    np.testing.assert_array_equal(a.get_velocity(), b.get_velocity())
+    for c in ctxs:
+        c.close()
