@@ -60,7 +60,7 @@ struct SceneDev {
     const float4* X;    // rest positions
     const int* topo;    // n_elements * NE
     const float4* eq;   // n_elements * NQ * 3
-    const int4* slots;  // n_nodes, colour-sorted: node, first owner, owner count, 0
+    const int4* slots;  // n_nodes, colour-sorted: node, first owner, owner count, 1 if the node is ever fixed
     const int* owners;  // packed (eid << 5) | r
     const int* fixed;   // n_fixed node ids
     const int* fixed_group;            // n_fixed rigid-group indices
@@ -125,8 +125,10 @@ struct alignas(16) VWork {
 constexpr int kIdBits = 27;
 constexpr int kIdMask = (1 << kIdBits) - 1;
 constexpr int kSpareBits = 32 - kIdBits;
+constexpr int kEntryFixed = 1 << kOwnerShift;
 template <int NE> struct EntryLayout {
-    // node ids, then r, then the record index; padded to a multiple of 4 words
+    // node ids, then r (with kEntryFixed in the entries of the point lanes, NE > 10, if the vertex is
+    // ever fixed), then the record index; padded to a multiple of 4 words
     static constexpr int kIds = 0, kR = NE, kRec = NE + 1;
     static constexpr int kWords = ((NE + 2) + 3) / 4 * 4;
     static constexpr long long kMaxRecords = 1ll << 31;

@@ -482,6 +482,7 @@ __device__ __forceinline__ unsigned entry_spare(const float* en, int i) { return
 template <int NE> __device__ __forceinline__ int entry_r(const float* en) {
     if constexpr (NE == 4) return 0;   // own node first
     else if constexpr (NE == 8) return (int)entry_spare(en, 0);
+    else if constexpr (NE > 10) return __float_as_int(en[EntryLayout<NE>::kR]) & (kEntryFixed - 1);
     else return __float_as_int(en[EntryLayout<NE>::kR]);
 }
 template <int NE> __device__ __forceinline__ int entry_rec(const float* en) {
@@ -802,7 +803,7 @@ k_vertex_points(const SceneDev* __restrict__ scenes, const VWork* __restrict__ w
     const bool on = g < GW;   // Q2: five lanes of a warp have no pair
     const int slot = (threadIdx.x >> 5) * GW + (on ? g : 0);
     const unsigned long long keep = policy_keep(), stream = policy_stream();
-    int scene, count, pair_base, n_pairs, r, rec, ids[NI];
+    int scene, count, pair_base, n_pairs, r, rec, fixed, ids[NI];   // fixed: the pair's vertex if it is ever fixed, else -1
     int4 vertex;   // of this pair slot's vertex: node, first owner, owner count
     auto fetch_pair = [&](const SceneDev& S, int p) {
         const int* en = reinterpret_cast<const int*>(S.ent) + (size_t)(pair_base + p) * EW;
@@ -811,6 +812,8 @@ k_vertex_points(const SceneDev* __restrict__ scenes, const VWork* __restrict__ w
         for (int k = 0; k < NI; ++k) ids[k] = has && j + k * LP < NE ? ld_hint(en + j + k * LP, stream) & kIdMask : 0;
         r = has ? ld_hint(en + NE, stream) : 0;
         rec = has ? ld_hint(en + NE + 1, stream) : 0;
+        fixed = r & kEntryFixed ? ld_hint(en + (r & (kEntryFixed - 1)), stream) & kIdMask : -1;
+        r &= kEntryFixed - 1;
     };
     auto fetch = [&](int w) {   // static data of item w, up to its first round's node ids
         const VWork wk = work[w];
@@ -861,8 +864,8 @@ k_vertex_points(const SceneDev* __restrict__ scenes, const VWork* __restrict__ w
 #pragma unroll
         for (int k = 0; k < NC; ++k) { sum[k] = 0.f; cmp[k] = 0.f; }
         for (int base = 0; base < n_pairs; base += SLOTS) {
-            const bool has = on && base + slot < n_pairs;
             if (base) fetch_pair(S, base + slot);
+            const bool has = on && base + slot < n_pairs && (fixed < 0 || S.mask[fixed] != 0);
             float acc[9];
 #pragma unroll
             for (int k = 0; k < 9; ++k) acc[k] = 0.f;
@@ -1017,7 +1020,10 @@ template <int E> struct LaneMinBlocks {
 // scene pointers, vertex slot, owner entry, node displacements, then the solve's own state.  All
 // of it up to the first owner entry is data that no kernel of a step writes, so it is loaded
 // before pdl_wait(), under the previous colour's tail; after the wait only the gathers, the
-// arithmetic and the store are left.  The slot (node, first owner, owner count) is one 16-byte
+// arithmetic and the store are left.  A vertex that is never fixed starts on its owners before its
+// mask is known; one that is, masked in all but its first sub-step, waits for it and skips them (a
+// sweep of 24 P1 scenes of 18,785 nodes, fixed but for their tip, 0.30 -> 0.23 ms; six Q2 scenes of
+// 21,609 nodes 1.29 -> 0.99).  The slot (node, first owner, owner count) is one 16-byte
 // load, and in a launch of one item per block the state the solve needs is prefetched into L1
 // while the owners are evaluated (launches of several waves hide it behind other warps, and their
 // L1 path is what binds them: 256 scenes 173.8 ms per frame with it, 167.4 without).
@@ -1031,7 +1037,7 @@ __global__ void __launch_bounds__(kBlock, LaneMinBlocks<E>::value) k_vertex(cons
     const int lane = threadIdx.x & 31;
     const unsigned long long stream = policy_stream();
     int scene, t, glane, o, oe, vid;
-    bool valid;
+    bool valid, fixed;
     float4 nxt[EW / 4];
     auto fetch = [&](int w) {   // this lane's part of item w, up to its first owner entry
         const int4 wk = __ldg(reinterpret_cast<const int4*>(work + w));   // scene, slot_begin, count, lanes
@@ -1043,6 +1049,7 @@ __global__ void __launch_bounds__(kBlock, LaneMinBlocks<E>::value) k_vertex(cons
         valid = group < wk.z;
         const int4 sl = valid ? __ldg(S.slots + wk.y + group) : make_int4(0, 0, 0, 0);
         vid = sl.x;
+        fixed = sl.w != 0;
         o = sl.y + glane;
         oe = sl.y + sl.z;
         if (S.ent && o < oe) {
@@ -1058,6 +1065,7 @@ __global__ void __launch_bounds__(kBlock, LaneMinBlocks<E>::value) k_vertex(cons
     while (true) {
         const SceneDev& S = scenes[scene];
         const bool active = valid && S.mask[vid] != 0;
+        if (fixed && !active) o = oe;   // only the ever fixed wait for their mask before the owners
         if (alone && active && glane == 0) {
             asm volatile("prefetch.global.L1 [%0];" ::"l"(S.u_last + vid));
             asm volatile("prefetch.global.L1 [%0];" ::"l"(S.y + vid));
@@ -1320,9 +1328,10 @@ k_vbd_substep(const SceneDev* __restrict__ scene, const VWork* __restrict__ work
     const int node0 = blockIdx.x * blockDim.x + threadIdx.x, nodes = gridDim.x * blockDim.x;
     const bool mixed = S.precision != 0, cheb = rho > 0.f;
     int t = 1, glane = 0, o = 0, oe = 0, vid = -1;   // this lane's part of its next item
+    bool fixed = false;
     float4 nxt[EW / 4];
     auto fetch = [&](int w, int end) {
-        vid = -1; o = oe = 0; t = 1; glane = 0;
+        vid = -1; o = oe = 0; t = 1; glane = 0; fixed = false;
         if (w >= end) return;
         const int4 wk = __ldg(reinterpret_cast<const int4*>(work + w));   // scene, slot_begin, count, lanes
         t = wk.w;
@@ -1331,6 +1340,7 @@ k_vbd_substep(const SceneDev* __restrict__ scene, const VWork* __restrict__ work
         if (group >= wk.z) return;
         const int4 sl = __ldg(S.slots + wk.y + group);
         vid = sl.x;
+        fixed = sl.w != 0;
         o = sl.y + glane;
         oe = sl.y + sl.z;
         if (o < oe) {
@@ -1352,6 +1362,7 @@ k_vbd_substep(const SceneDev* __restrict__ scene, const VWork* __restrict__ work
             for (int w = c_begin + first; w < c_end; w += step) {   // sub-block-uniform
                 if (w != c_begin + first) fetch(w, c_end);
                 const bool active = vid >= 0 && S.mask[vid] != 0;
+                if (fixed && !active) o = oe;
                 if (active && glane == 0) {
                     asm volatile("prefetch.global.L1 [%0];" ::"l"(S.u_last + vid));
                     asm volatile("prefetch.global.L1 [%0];" ::"l"(S.y + vid));

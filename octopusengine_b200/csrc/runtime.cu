@@ -188,6 +188,7 @@ struct oct_scene {
     std::vector<int32_t> own_off;                    // owner CSR offsets in slot order (host copy)
     std::vector<float> masses, X;
     std::vector<int32_t> fixed, fixed_group;
+    std::vector<int32_t> masked;    // of a linear level: its nodes that the full level fixes
     float fix_host[kFixGroups * 16] = {0};
     float* d_fix = nullptr;
     // device
@@ -531,6 +532,7 @@ oct_status build_multigrid(oct_ctx* c, const oct_scene_desc* d, oct_scene* s) {
     dl.threads_per_vertex = 0;
     dl.mg_linear = 0.f;
     auto* sub = new oct_scene();
+    for (int32_t id : s->fixed) if (compact[id] >= 0) sub->masked.push_back(compact[id]);
     oct_status st = build_scene(c, &dl, sub);
     if (st) { sub->mem.release(); delete sub; return st; }
     s->mg_sub = sub;
@@ -842,8 +844,12 @@ oct_status build_scene(oct_ctx* c, const oct_scene_desc* d, oct_scene* s) {
     if ((st = upload(c, s->mem, maskd, mask)) || (st = upload(c, s->mem, topod, topo)) || (st = upload(c, s->mem, eqd, eq)) ||
         (st = upload(c, s->mem, ownd, owners)))
         return st;
+    std::vector<char> ever_fixed(N, 0);
+    for (int32_t id : s->fixed) ever_fixed[id] = 1;
+    for (int32_t id : s->masked) ever_fixed[id] = 1;
     std::vector<int4> slots(N);
-    for (int sl = 0; sl < N; ++sl) slots[sl] = make_int4(slot_vids[sl], own_off[sl], own_off[sl + 1] - own_off[sl], 0);
+    for (int sl = 0; sl < N; ++sl)
+        slots[sl] = make_int4(slot_vids[sl], own_off[sl], own_off[sl + 1] - own_off[sl], ever_fixed[slot_vids[sl]]);
     int4* slotd;
     if ((st = upload(c, s->mem, slotd, slots))) return st;
     h.slots = slotd;
@@ -949,7 +955,7 @@ oct_status build_scene(oct_ctx* c, const oct_scene_desc* d, oct_scene* s) {
                 for (int j = 1; j < 8; ++j)
                     ei[j] |= (int32_t)((((uint64_t)(uint32_t)rec) >> (kSpareBits * (j - 1))) & ((1u << kSpareBits) - 1)) << kIdBits;
             } else {
-                ei[NE] = r;
+                ei[NE] = r | (NE > 10 && ever_fixed[te[r]] ? kEntryFixed : 0);
                 ei[NE + 1] = rec;
             }
         }
