@@ -483,6 +483,7 @@ oct_status copy_out(oct_ctx* c, void* out, const void* d, size_t bytes) {
 
 // Vertex work items of every colour for the scene's lane mapping (tpv), uploaded to the device.
 oct_status build_vertex_work(oct_scene* s) {
+    if (s->solver != OCT_SOLVER_VBD) return OCT_OK;   // the vertex kernels alone read it
     std::vector<VWork> vw;
     s->vwork_off.assign(1, 0);
     s->form.clear();
@@ -1311,13 +1312,16 @@ oct_status oct_scene_footprint(const oct_scene_desc* d, size_t* bytes) {
     const size_t N = d->n_nodes, E = d->n_elements;
     size_t b = N * (7 * sizeof(float4) + 3 * sizeof(int)) + (d->rho > 0.f ? 2 * N * sizeof(float4) : 0);
     b += E * ne * sizeof(int) * 2 + E * nq * 3 * sizeof(float4);   // topology, owners, quadrature records
-    b += E * ne * (size_t)entry_words(ne) * sizeof(float);                  // owner entries
-    b += (ne == 4 ? 4 : 1) * E * 3 * sizeof(float4);                        // distinct records, at most
+    if (d->solver == OCT_SOLVER_VBD) {
+        b += E * ne * (size_t)entry_words(ne) * sizeof(float);              // owner entries
+        b += (ne == 4 ? 4 : 1) * E * 3 * sizeof(float4);                    // distinct records, at most
+        b += (N / 4 + E * ne / 12 + 64) * sizeof(VWork);                    // work items, of 4 vertices or 12 pairs at least
+    }
     if (d->solver == OCT_SOLVER_EXPLICIT) b += E * ne * (sizeof(float4) + 2 * sizeof(int));   // contributions, their places, topology
     if (d->solver != OCT_SOLVER_XPBD) b += N * sizeof(int);                                   // fixation map
-    b += (N / 16 + 64) * sizeof(VWork) + (N / 256 + 8) * 2 * sizeof(NWork) + (size_t)std::max(d->n_fixed, 0) * sizeof(int);
-    if (d->solver == OCT_SOLVER_XPBD) b += E * (ne + 1) * sizeof(int);   // colour-sorted element ids and topology
-    b += 4096;   // descriptors and reduction scratch
+    b += (N / 256 + 8) * 2 * sizeof(NWork) + (size_t)std::max(d->n_fixed, 0) * sizeof(int);
+    if (d->solver == OCT_SOLVER_XPBD) b += E * (ne + 1) * sizeof(int) + (E / 2 + 64) * sizeof(XWork);   // colour-sorted element ids and topology
+    b += 8192;   // descriptors, reduction scratch, and what rounding to 256 bytes adds
     *bytes = b;
     return OCT_OK;
 }
