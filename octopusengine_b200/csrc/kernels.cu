@@ -1026,7 +1026,8 @@ template <int E> struct LaneMinBlocks {
 // 21,609 nodes 1.29 -> 0.99).  The slot (node, first owner, owner count) is one 16-byte
 // load, and in a launch of one item per block the state the solve needs is prefetched into L1
 // while the owners are evaluated (launches of several waves hide it behind other warps, and their
-// L1 path is what binds them: 256 scenes 173.8 ms per frame with it, 167.4 without).
+// L1 path is what binds them: 256 scenes, in turns on one GPU, 173.8 ms per frame with it and 167.4
+// without, 170.7 before either; other GPUs of the kind gave 171.4 without).
 template <int E, int MAT>
 __global__ void __launch_bounds__(kBlock, LaneMinBlocks<E>::value) k_vertex(const SceneDev* __restrict__ scenes, const VWork* __restrict__ work,
                                                    int n_work, int mode, StepParams P, double* red) {
@@ -1979,7 +1980,8 @@ template <int E, int MAT>
 __global__ void __launch_bounds__(kBlock) k_explicit_elem(const SceneDev* __restrict__ scenes, int n_elements,
                                                           float4* __restrict__ contrib, StepParams P) {
     // contributions go to the owner's place in slot order (SceneDev::owner_at), read in order by
-    // k_explicit_gather
+    // k_explicit_gather.  P1, Q1 and P2 come here only with damping (k_explicit_thread)
+    constexpr bool undamped = E == 8 || E == 9;
     constexpr int NE = ElemT<E>::NE, NQ = ElemT<E>::NQ, G = ElemLanes<E>::G, GPB = kBlock / G;
     constexpr int NI = (NE + G - 1) / G;   // nodes per lane
     static_assert(NQ <= G, "one quadrature point per lane");
@@ -2020,7 +2022,7 @@ __global__ void __launch_bounds__(kBlock) k_explicit_elem(const SceneDev* __rest
         V3 F1 = J0 * m1.x + J1 * m1.y + J2 * m1.z;
         V3 F2 = J0 * m2.x + J1 * m2.y + J2 * m2.z;
         F0.x += 1.f; F1.y += 1.f; F2.z += 1.f;
-        if (S.damping == 0.f) {   // without damping only -V P g is needed: P~ once per point
+        if (undamped && S.damping == 0.f) {   // without damping only -V P g is needed: P~ once per point
             pk1_tilde<MAT>(F0, F1, F2, C.z, C.w, C.y * wq<E>(q), m0, m1, m2, F0, F1, F2);
         }
         s_F[grp][q][0] = make_float4(F0.x, F0.y, F0.z, 0.f);
@@ -2032,7 +2034,7 @@ __global__ void __launch_bounds__(kBlock) k_explicit_elem(const SceneDev* __rest
     }
     __syncwarp();
     const float kd = S.damping;
-    if (kd == 0.f) {   // f_i = -sum_q P~_q dN_qi
+    if (undamped && kd == 0.f) {   // f_i = -sum_q P~_q dN_qi
 #pragma unroll
         for (int k = 0; k < NI; ++k) {
             const int i = lane + k * G;
