@@ -51,3 +51,10 @@ def test_explicit(ctx, element, material, cells):
 def test_xpbd(ctx, element, cells, material):
     _check(ctx, "xpbd", element, cells, material, False, 2, 1 / 120)
     _check(ctx, "xpbd", element, cells, material, True, 2, 1 / 120)
+
+
+@pytest.mark.parametrize("cells", CELLS[:3])
+@pytest.mark.parametrize("element", [O.TETRA, O.HEXA, O.TETRA10, O.TETRA20, O.HEXA27])
+def test_explicit_damped(ctx, element, cells):
+    _check(ctx, "explicit", element, cells, O.STABLE_NEOHOOKE, False, 20, 20 * 2e-5, damping=1e-4)
+    _check(ctx, "explicit", element, cells, O.NEOHOOKE, True, 20, 20 * 2e-5, precision=1, damping=1e-4)
