@@ -478,6 +478,7 @@ bool pageable(const void* p) {
 oct_status copy_out(oct_ctx* c, void* out, const void* d, size_t bytes) {
     OCT_CUDA(c, cudaMemcpyAsync(out, d, bytes, cudaMemcpyDeviceToHost, c->stream));
     OCT_CUDA(c, cudaStreamSynchronize(c->stream));
+    hold(c, 0);
     return OCT_OK;
 }
 
@@ -1198,6 +1199,7 @@ oct_status read_nodes(oct_scene* s, const float4* d, float* out, bool add_rest) 
         if (io.p) {
             launch_nodes_out(d, add_rest ? s->h.X : nullptr, (float*)io.p, s->n_nodes, c->stream);
             OCT_CUDA(c, cudaStreamSynchronize(c->stream));
+            hold(c, 0);
             std::memcpy(out, io.p, bytes);
             return OCT_OK;
         }

@@ -65,6 +65,9 @@ def test_a_context_gives_way_to_one_in_flight(built):
     assert launches(b) > 3
     a.sync()
     assert launches(b) == 3
+    a.step(1 / 60, 3, sync=False)
+    a.get_position()   # waits for the frame, too
+    assert launches(b) == 3
     a.step(1 / 60, 3)
     np.testing.assert_array_equal(a.get_position(), b.get_position())
     np.testing.assert_array_equal(a.get_velocity(), b.get_velocity())
