@@ -10,7 +10,8 @@ Synthetic data; the state (~1 GB) is larger than L2, so no flush is needed betwe
 
 metric: vertex-iterations/s = sum over scenes of free nodes x iterations x sub-steps per
 step, / time.  Also reported: the plain single-scene drop-in path (each scene stepped on
-its own, FP32, one launch per colour, no graph) on the same scenes and GPU, p50/p99 step
+its own, FP32, no graph: a small or medium scene's sub-step in one launch, else one launch per
+colour) on the same scenes and GPU, p50/p99 step
 latency, the end-to-end number through the C ABI with host buffers, the roofline of the
 dominant kernel (algorithmic flops and bytes of the reference algorithm: Jx, F, dF/dx, PK1,
 the six symmetric Hessian blocks and their assembly; the executed-flop rate beside them), the reference CPU VBD path timed on the host cores (one thread, as the reference runs;
@@ -977,7 +978,8 @@ def main():
         torch.cuda.synchronize()
         plain_ms = p0.elapsed_time(p1)
         plain = {"value": vit_per_step / (plain_ms * 1e-3), "unit": "vertex-iter/s", "ms_per_step": plain_ms,
-                 "path": "each scene stepped alone through oct_scene_step: FP32, one launch per colour, no graph"}
+                 "path": "each scene stepped alone through oct_scene_step: FP32, no graph; a small or medium "
+                         "scene's sub-step in one launch, else one launch per colour"}
 
     # ---- the rest of the metric on the same GPU: config 2 alone, and a short served stream
     p2_line, served_line, xpbd_line, cube_lines = None, None, None, None
