@@ -1317,7 +1317,8 @@ oct_status oct_scene_footprint(const oct_scene_desc* d, size_t* bytes) {
     if (d->solver == OCT_SOLVER_VBD) {
         b += E * ne * (size_t)entry_words(ne) * sizeof(float);              // owner entries
         b += (ne == 4 ? 4 : 1) * E * 3 * sizeof(float4);                    // distinct records, at most
-        b += (N / 4 + E * ne / 12 + 64) * sizeof(VWork);                    // work items, of 4 vertices or 12 pairs at least
+        const bool packed = ne > 10 || d->threads_per_vertex < 0;           // work items, of 4 vertices or 12 pairs at least
+        b += (packed ? std::max(N / 4, E * ne / 12) : N / 4) * sizeof(VWork) + 64 * sizeof(VWork);
     }
     if (d->solver == OCT_SOLVER_EXPLICIT) b += E * ne * (sizeof(float4) + 2 * sizeof(int));   // contributions, their places, topology
     if (d->solver != OCT_SOLVER_XPBD) b += N * sizeof(int);                                   // fixation map

@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 ELEMENTS = [(O.TETRA, (9, 5, 4)), (O.HEXA, (12, 7, 6)), (O.TETRA10, (7, 4, 3)), (O.TETRA20, (5, 3, 3)), (O.HEXA27, (6, 4, 4))]
 
 
-@pytest.mark.parametrize("lanes", [0, 1, 32])
+@pytest.mark.parametrize("lanes", [0, -1, 1, 32])
 @pytest.mark.parametrize("distorted", [False, True])
 @pytest.mark.parametrize("element,cells", ELEMENTS)
 @pytest.mark.parametrize("solver", ["vbd", "xpbd", "explicit"])
