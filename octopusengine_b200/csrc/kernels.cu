@@ -1022,8 +1022,8 @@ template <int E> struct LaneMinBlocks {
 // before pdl_wait(), under the previous colour's tail; after the wait only the gathers, the
 // arithmetic and the store are left.  A vertex that is never fixed starts on its owners before its
 // mask is known; one that is, masked in all but its first sub-step, waits for it and skips them (a
-// sweep of 24 P1 scenes of 18,785 nodes, fixed but for their tip, 0.30 -> 0.23 ms; six Q2 scenes of
-// 21,609 nodes 1.29 -> 0.99).  The slot (node, first owner, owner count) is one 16-byte
+// sweep of 24 P1 scenes of 18,785 nodes, fixed but for their tip, 100 -> 75 us; six Q2 scenes of
+// 21,609 nodes 437 -> 325).  The slot (node, first owner, owner count) is one 16-byte
 // load, and in a launch of one item per block the state the solve needs is prefetched into L1
 // while the owners are evaluated (launches of several waves hide it behind other warps, and their
 // L1 path is what binds them: 256 scenes, in turns on one GPU, 173.8 ms per frame with it and 167.4
